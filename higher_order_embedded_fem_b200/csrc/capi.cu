@@ -659,9 +659,8 @@ int hoefem_cg_solve_mixed(hoefem_model m, const double* system_values, hoefem_pr
   w.stream_ms_total = 0.0;
   View A(system_values, mm.nnz, mem, mm.stream, true);
   View B(b, mm.ndof, mem, mm.stream, true), X(x, mm.ndof, mem, mm.stream, true);
-  DBuf<float> A32;
-  A32.alloc(mm.nnz);
-  to_f32(A.d, A32.p, mm.nnz, mm.stream);
+  if (w.A32.n < (size_t)mm.nnz) w.A32.alloc(mm.nnz);
+  to_f32(A.d, w.A32.p, mm.nnz, mm.stream);
   if (p && p->p.kind == PREC_SCHWARZ && p->p.ready && (!p->p.vals32.p || !p->p.want_fp32)) {
     p->p.want_fp32 = true;
     precond_to_fp32(p->p, mm.stream);
@@ -669,7 +668,7 @@ int hoefem_cg_solve_mixed(hoefem_model m, const double* system_values, hoefem_pr
   HOEFEM_CUDA(cudaMemcpyAsync(w.b.p, B.d, mm.ndof * sizeof(double), cudaMemcpyDeviceToDevice, mm.stream));
   HOEFEM_CUDA(cudaMemcpyAsync(w.x.p, X.d, mm.ndof * sizeof(double), cudaMemcpyDeviceToDevice, mm.stream));
   i64 it = 0, replacements = 0;
-  int st = cg_solve_reliable(w, A.d, A32.p, p ? &p->p : nullptr, tol, max_iter, delta, &it, &replacements, mm.stream);
+  int st = cg_solve_reliable(w, A.d, w.A32.p, p ? &p->p : nullptr, tol, max_iter, delta, &it, &replacements, mm.stream);
   HOEFEM_CUDA(cudaMemcpyAsync(X.d, w.x.p, mm.ndof * sizeof(double), cudaMemcpyDeviceToDevice, mm.stream));
   X.copy_out();
   sync(mm);

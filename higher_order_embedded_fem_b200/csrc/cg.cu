@@ -1,4 +1,7 @@
-// Preconditioned conjugate gradient on the device.
+// Preconditioned conjugate gradient on the device: the solve's set-up, residual
+// replacement and engine choice, and the graphs of kernel chunks that run the
+// iterations where the persistent kernels (cg_persist.cu, cg_stream.cu) do
+// not apply.
 //
 // Reference: ConjugateGradient::solve_with_guess_ (fenris/src/cg.rs:376-482)
 // with RelativeResidualCriterion (cg.rs:77-124).  The loop control lives on
@@ -768,15 +771,21 @@ int run_pcg(CgWork& w, Operator A, const Precond* P, bool p32, double tol, i64 m
     et.us_per_it[engine] = 1e3 * ms / (double)n_it;
     if (++et.phase == 4) et.choice = et.us_per_it[1] < et.us_per_it[0] ? 1 : 0;
   };
-  if (streamed) {
+  const void* vals = f32 ? (const void*)A.v32 : (const void*)A.v64;
+  if (streamed || cg_persist_usable(w, vals, f32, P, p32, s)) {
+    // one launch per residual replacement
     cg_stream_arm(w, A64 ? delta : 0.0, s);
     w.stream_ms = 0.f;
     const i64 cap_s = max_iter >= 0 ? max_iter : 10 * (i64)n;
     i64 nrep_s = 0;
     for (;;) {
       const i64 it0 = w.h_st->iters;
-      cg_stream_iterate(w, f32, P, p32, A64 != nullptr, s);
-      w.stream_iterations += w.h_st->iters - it0;
+      if (streamed) {
+        cg_stream_iterate(w, f32, P, p32, A64 != nullptr, s);
+        w.stream_iterations += w.h_st->iters - it0;
+      } else {
+        cg_persist_iterate(w, vals, f32, P, p32, A64 != nullptr, s);
+      }
       // a launch that ran no iteration found the solve finished by the
       // replacement before it
       const bool ran = w.h_st->iters > it0;
@@ -812,7 +821,7 @@ int run_pcg(CgWork& w, Operator A, const Precond* P, bool p32, double tol, i64 m
         return HOEFEM_CG_MAX_ITERATIONS;
       }
     }
-    sample(1);
+    sample(streamed ? 1 : 0);
     if (replacements) *replacements = nrep_s;
     *iters = w.h_st->iters;
     return w.h_st->status;

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "hoefem.h"
+#include "pcg_layout.h"
 
 namespace hoefem {
 
@@ -68,6 +69,13 @@ struct DBuf {
     if (count) HOEFEM_CUDA(cudaMemcpyAsync(p, h, count * sizeof(T), cudaMemcpyHostToDevice, s));
   }
   void upload(const std::vector<T>& h, cudaStream_t s) { upload(h.data(), h.size(), s); }
+  // with 16 readable bytes behind the data (bulk copies read whole 16-byte
+  // granules)
+  void upload_padded(const std::vector<T>& h, cudaStream_t s) {
+    alloc(h.size() + 16 / sizeof(T));
+    zero(s);
+    if (!h.empty()) HOEFEM_CUDA(cudaMemcpyAsync(p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, s));
+  }
   void zero(cudaStream_t s) {
     if (n) HOEFEM_CUDA(cudaMemsetAsync(p, 0, n * sizeof(T), s));
   }
@@ -149,6 +157,15 @@ struct Block {
 // rest), staged CUDA-core kernels only, or the colored scatter kernels.
 enum StiffnessPath { STIFFNESS_AUTO = 0, STIFFNESS_CUDA_CORES = 1, STIFFNESS_STAGED = 2 };
 
+// Tiles of the persistent CG (cg_persist.cu) for one value size.
+struct PcgOpLayout {
+  int state = 0;  // 0 not built, 1 built, -1 a node's rows do not fit a stage
+  int grid = 0, max_blk = 0;
+  long long cap = 0;  // value bytes of a tile
+  DBuf<PcgTile> tiles;
+  DBuf<int> cta;  // grid + 1
+};
+
 struct Model {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -171,6 +188,7 @@ struct Model {
   int spmv_lanes32 = 0;   // SpMV variant for FP32 values (0: as spmv_lanes)
   bool spmv_pinned = false;  // set explicitly by the caller: no autotuning
   int stiffness_path = STIFFNESS_AUTO;
+  PcgOpLayout pcg[2];  // FP64, FP32 values
   NodeRows rows() const;
   ~Model();
 };

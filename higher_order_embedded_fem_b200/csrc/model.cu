@@ -201,8 +201,8 @@ void ensure_device(Model& m) {
   if (!m.stream) HOEFEM_CUDA(cudaStreamCreateWithFlags(&m.stream, cudaStreamNonBlocking));
   cudaStream_t s = m.stream;
   m.d_X.upload(m.X, s);
-  m.d_adj_off.upload(m.adj_off, s);
-  m.d_adj.upload(m.adj, s);
+  m.d_adj_off.upload_padded(m.adj_off, s);
+  m.d_adj.upload_padded(m.adj, s);
   m.d_diag_slot.upload(m.diag_slot, s);
   m.d_base.upload(m.base, s);
   m.d_err.alloc(1);

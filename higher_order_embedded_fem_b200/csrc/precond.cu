@@ -466,7 +466,7 @@ void precond_create_schwarz(Precond& p, const i64* sub_off, const i64* sub_nodes
   std::vector<int> so(p.sub_off.begin(), p.sub_off.end()), sn(p.sub_nodes.begin(), p.sub_nodes.end());
   std::vector<int> un(p.untreated.begin(), p.untreated.end());
   p.d_sub_off.upload(so, st);
-  p.d_sub_nodes.upload(sn, st);
+  p.d_sub_nodes.upload_padded(sn, st);
   p.d_untreated.upload(un, st);
   // rows with subdomain entries (or none at all) are visited by the row
   // kernels; the untreated nodes are applied elementwise
@@ -496,9 +496,10 @@ void precond_create_schwarz(Precond& p, const i64* sub_off, const i64* sub_nodes
     for (i64 s = 0; s < nsub; ++s)
       for (i64 k = sub_off[s]; k < sub_off[s + 1]; ++k) slot[k] = fill[sub_nodes[k]]++;
     p.d_npair_off.upload(poff, st);
-    p.d_npair.upload(slot, st);
+    p.d_npair.upload_padded(slot, st);
     p.ysub.alloc(3 * sub_off[nsub]);
-    p.bsym.alloc(stage_off[nsub]);
+    p.bsym.alloc(stage_off[nsub] + 4);  // whole 16-byte granules (bulk copies)
+    p.bsym.zero(st);
     p.block_apply = 3 * p.max_nodes <= 96;  // one thread per block row
   }
   p.vals.alloc(p.nnz);

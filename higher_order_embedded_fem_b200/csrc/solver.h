@@ -10,6 +10,14 @@ namespace hoefem {
 
 enum PrecondKind { PREC_NONE = 0, PREC_DIAGONAL = 1, PREC_SCHWARZ = 2 };
 
+// Row tiles of the Schwarz blocks for the persistent CG, one value size.
+struct PcgSwLayout {
+  long long cap = 0;
+  int grid = 0;
+  DBuf<PcgSwTile> tiles;
+  DBuf<int> cta;  // grid + 1
+};
+
 struct Precond {
   int kind = PREC_DIAGONAL;
   Model* m = nullptr;
@@ -54,6 +62,7 @@ struct Precond {
   DBuf<double> ysub;
   DBuf<int> d_npair_off;  // nv + 1: a node's slots in ysub (3 entries each)
   DBuf<int> d_npair;      // slot of every (subdomain, node) incidence (sub_nodes order)
+  PcgSwLayout pcg[2];     // FP64, FP32 blocks
   NodeRows rows() const;
 };
 
@@ -158,6 +167,11 @@ struct CgWork {
   // FP32 copy of the search direction (one 16-byte entry per node) for the
   // FP32 operator products of the mixed form's chunked engine
   DBuf<float4> p32;
+  DBuf<float> A32;  // FP32 copy of a caller's matrix (hoefem_cg_solve_mixed)
+  // persistent CG: FP64 search direction with one 32-byte entry per node, the
+  // counter of its grid barriers and their partial sums
+  DBuf<double> p64, ppart;
+  DBuf<unsigned> pbar;
   DBuf<CgState> st;
   DBuf<unsigned> counter;
   CgState* h_st = nullptr;  // pinned
@@ -245,6 +259,13 @@ struct Learned;
 // count the iterations with and without the correction.
 int cg_solve_learned(CgWork& w, const double* vals, const Precond* P, Learned* L, double tol, i64 max_iter,
                      i64* iters, i64* kept, i64* dropped, cudaStream_t s);
+
+// Persistent CG on the CSR values in place (cg_persist.cu): whether it takes
+// this solve (layouts built on first use), and one launch with the contract of
+// cg_stream_iterate.
+bool cg_persist_usable(CgWork& w, const void* vals, bool f32, const Precond* P, bool p32, cudaStream_t s);
+void cg_persist_iterate(CgWork& w, const void* vals, bool f32, const Precond* P, bool p32, bool reliable,
+                        cudaStream_t s);
 
 // Streamed CG (cg_stream.cu).  cg_stream_usable: whether the persistent
 // kernel can run this solve; cg_stream_prepare packs the operator (FP64

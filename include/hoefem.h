@@ -352,17 +352,21 @@ typedef enum { HOEFEM_PRECISION_FP64 = 0, HOEFEM_PRECISION_MIXED = 1 } hoefem_pr
 int hoefem_integrator_set_precision(hoefem_integrator it, int precision, double delta);
 /* CG engine of the integrator's Jacobian solves and of hoefem_cg_solve /
    hoefem_cg_solve_mixed on a model (no counterpart in the reference, whose CG
-   is one host loop).  Two engines run the same recurrence: CUDA graphs of
-   kernel chunks, and the persistent streamed CG (one cooperative launch per
-   solve, the operator and the Schwarz blocks streamed through shared memory;
-   for no preconditioner, diagonal, or Schwarz with subdomains of at most 27
-   nodes).  HOEFEM_CG_ENGINE_AUTO (default): models with fewer than 32,768
-   nodes use the graphs; for larger ones, per operator precision and
-   preconditioner kind, each engine's first solve sets it up (graphs, stream
-   layouts) and its next solve of at least 20 iterations is timed whole
+   is one host loop).  Two engines run the same recurrence: the chunked engine
+   on the CSR values in place (one cooperative launch per residual
+   replacement; CUDA graphs of kernel chunks where that launch does not apply:
+   pinned SpMV variants, Schwarz as an assembled matrix, values not aligned to
+   16 bytes, nodes with more than 340 FP64 or 680 FP32 neighbours), and the
+   persistent streamed CG (one cooperative launch per solve, the operator and
+   the Schwarz blocks packed into stream layouts; for no preconditioner,
+   diagonal, or Schwarz with subdomains of at most 27 nodes).
+   HOEFEM_CG_ENGINE_AUTO (default): models with fewer than 32,768 nodes use
+   the chunked engine; for larger ones, per operator precision and
+   preconditioner kind, each engine's first solve sets it up (tiles, graphs,
+   stream layouts) and its next solve of at least 20 iterations is timed whole
    (the solve's set-up, value packing, residual replacements and launches
    included); the engine with the lower time per iteration is kept; HOEFEM_CG_ENGINE_CHUNKED:
-   always the graphs; HOEFEM_CG_ENGINE_STREAMED: the streamed CG or
+   always the chunked engine; HOEFEM_CG_ENGINE_STREAMED: the streamed CG or
    HOEFEM_ERR_INVALID_ARGUMENT.  options (bit mask):
    HOEFEM_CG_SCHWARZ_FP16: in the mixed-precision form the streamed CG keeps
    the Schwarz blocks in FP16 scaled by each block's largest magnitude;
