@@ -734,6 +734,7 @@ void launch_stiffness(const Model& m, const MatDev& mat, const double* u, double
       void* pb = stiffness_pair_buffer(m, *bp, f32, s);
       if (bp->kind == HOEFEM_ELEM_TET10) {
         if (f32) launch_stiffness_kind<10, float>(m, *bp, mat, u, nullptr, s, nullptr, (float*)pb);
+        else if (stiffness_moments_eligible(*bp)) launch_stiffness_moments(m, *bp, mat, u, (double*)pb, s);
         else launch_stiffness_kind<10, double>(m, *bp, mat, u, nullptr, s, nullptr, (double*)pb);
       } else {
         if (f32) launch_stiffness_kind<27, float>(m, *bp, mat, u, nullptr, s, nullptr, (float*)pb);

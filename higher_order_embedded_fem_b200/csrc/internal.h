@@ -145,6 +145,7 @@ struct Block {
   mutable DBuf<int> d_tc_off, d_tc_ent;
   mutable DBuf<double> d_pb64;  // FP64 node-pair blocks of the staged CUDA-core path
   mutable DBuf<double> d_fst;   // staged element node forces
+  mutable DBuf<double> d_moment_w;  // per point: the weights of the tangent's moments (stiffness_moments.cu)
   mutable DBuf<int> d_noff, d_nent;  // per node: its (element, local node) incidences
   mutable int tc_nch = 0;
   mutable bool tc_ready = false, gmap_ready = false, nmap_ready = false;
@@ -220,6 +221,11 @@ void launch_stiffness_tc(const Model& m, const Block& blk, const MatDev& mat, co
 bool stiffness_pairs_eligible(const Model& m, const Block& blk);
 void* stiffness_pair_buffer(const Model& m, const Block& blk, bool f32, cudaStream_t s);
 void stiffness_gather_pairs(const Model& m, const Block& blk, bool f32, double* vals, bool assign, cudaStream_t s);
+// FP64 node-pair blocks of a Tet10 block with one rule, from moments of the
+// tangent (stiffness_moments.cu).
+bool stiffness_moments_eligible(const Block& blk);
+void launch_stiffness_moments(const Model& m, const Block& blk, const MatDev& mat, const double* u, double* pblk,
+                              cudaStream_t s);
 // Staged element forces of a whole block (same eligibility): the buffer
 // (element-major node forces) and the per-node gather adding into f.
 double* forces_stage_buffer(const Model& m, const Block& blk, cudaStream_t s);
