@@ -563,6 +563,7 @@ int hoefem_precond_set_block_apply(hoefem_precond p, int32_t on) {
   HOEFEM_REQUIRE(!on || 3 * p->p.max_nodes <= 96, HOEFEM_ERR_INVALID_ARGUMENT,
                  "block apply supports subdomains of at most 32 nodes");
   p->p.block_apply = on != 0;
+  p->p.apply_pinned = true;
   if (!on) precond_assemble(p->p, p->p.m->stream);  // the SpMV apply reads every entry
   API_END
 }

@@ -104,7 +104,7 @@ struct Args {
   unsigned* counter;  // grid barrier
   double* part;       // partial sums, 2 x MAX_SUMS x G
   int* err;
-  int reliable;
+  int reliable, chunk;  // residual replacements, at multiples of `chunk` iterations
   // shared memory
   int nw, stages, val_bytes, adj_bytes;  // warps that take tiles, ring stages and their parts
 };
@@ -617,7 +617,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_pcg(const Args A) {
     } else {
       beta = zr / zTr;
       zTr = zr;
-      if (A.reliable && rr <= delta2 * rr_ref) replace = 1;
+      // at the ends of chunks, as the graphs
+      if (A.reliable && iters % A.chunk == 0 && rr <= delta2 * rr_ref) replace = 1;
     }
     const bool last = done || replace;
     // ---- phase 3: x, r, p of the CTA's nodes ----
@@ -714,14 +715,15 @@ int align16(long long b) { return (int)((b + 15) & ~15LL); }
 
 // Whether the persistent kernel takes this solve, with its layouts built on
 // first use.  It does not take: Schwarz preconditioners applied as an SpMV or
-// without blocks, SpMV variants pinned by the caller, solves that report every
+// without blocks, SpMV variants or a Schwarz apply pinned by the caller (the
+// graphs, where the two applies differ in nothing else), solves that report every
 // chunk of iterations, rows too long for a stage, values not aligned to 16
 // bytes (bulk copies), devices without cooperative launch.
 bool cg_persist_usable(CgWork& w, const void* vals, bool f32, const Precond* P, bool p32, cudaStream_t s) {
   Model& m = *w.m;
   if (w.on_chunk || m.spmv_pinned || m.nv == 0 || ((uintptr_t)vals & 15)) return false;
   const bool sw = P && P->kind == PREC_SCHWARZ;
-  if (sw && (!P->block_apply || P->nsub == 0 || 3 * P->max_nodes > 96)) return false;
+  if (sw && (!P->block_apply || P->apply_pinned || P->nsub == 0 || 3 * P->max_nodes > 96)) return false;
   int dev = 0, coop = 0;
   HOEFEM_CUDA(cudaGetDevice(&dev));
   HOEFEM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
@@ -812,6 +814,7 @@ void cg_persist_iterate(CgWork& w, const void* vals, bool f32, const Precond* P,
   a.part = w.ppart.p;
   a.err = w.serr.p;
   a.reliable = reliable ? 1 : 0;
+  a.chunk = w.chunk;
   a.val_bytes = align16(L.cap + 32);
   a.adj_bytes = std::max(align16(4LL * L.max_blk + 16), IDX_BYTES);
   // as many stages as fit; three quarters of them at work, the rest in flight

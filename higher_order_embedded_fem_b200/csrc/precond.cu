@@ -9,18 +9,19 @@
 // Schwarz update on the device, in three steps:
 //  1. k_schwarz_gj: one CTA per subdomain gathers its 3n x 3n principal block
 //     of the system matrix (element-to-nnz map, no searches) into registers
-//     (16 x 16 threads, each a T x T tile) and inverts it by Gauss-Jordan
-//     elimination without pivoting.  For a symmetric block every pivot is
+//     (one 9 x 9 tile per thread) and inverts it by Gauss-Jordan elimination
+//     without pivoting, a node at a time.  For a symmetric block every pivot is
 //     positive exactly when the block is positive definite; with
 //     ||A||_F ||A^-1||_F <= 1e12 (so lambda_min >= 1e-12 lambda_max) the
-//     reference's spectrum rule is the plain inverse, which is written to a
-//     staging buffer.  Blocks that fail either test are listed for
+//     reference's spectrum rule is the plain inverse, whose symmetric part is
+//     stored.  Blocks that fail either test are listed for
 //     k_schwarz_factor: a parallel cyclic Jacobi eigensolver in shared memory
 //     (round-robin ordering: m/2 disjoint rotations per round, rows then
 //     columns) that applies the spectrum rule (1/|lambda|, floor
-//     1e-12 max|lambda|) and writes the recomposed block V f(L) V^T.
+//     1e-12 max|lambda|) and stores the symmetric part of the recomposed block
+//     V f(L) V^T.
 //  2. k_schwarz_scatter: per subdomain color (greedy coloring of the subdomain
-//     node lists, as the reference), the staged blocks are added into the
+//     node lists, as the reference), on demand the blocks are added into the
 //     preconditioner's own CSR values, so every entry receives its
 //     contributions in color order without atomics.
 //  3. k_schwarz_untreated: scalar Jacobi 1/a_ii on the untreated nodes.
@@ -65,119 +66,167 @@ namespace {
 constexpr int FACTOR_TPB = 256;
 
 
+// Inverse of the symmetric positive definite 3 x 3 matrix p (row-major) from its
+// minors (one division).  False unless the leading minors are positive, that
+// is unless the three pivots the scalar elimination would meet are.
+__device__ __forceinline__ bool inv3_spd(const double* p, double (&o)[9]) {
+  o[0] = p[4] * p[8] - p[5] * p[7];
+  o[1] = p[2] * p[7] - p[1] * p[8];
+  o[2] = p[1] * p[5] - p[2] * p[4];
+  o[3] = p[5] * p[6] - p[3] * p[8];
+  o[4] = p[0] * p[8] - p[2] * p[6];
+  o[5] = p[2] * p[3] - p[0] * p[5];
+  o[6] = p[3] * p[7] - p[4] * p[6];
+  o[7] = p[1] * p[6] - p[0] * p[7];
+  o[8] = p[0] * p[4] - p[1] * p[3];
+  const double det = p[0] * o[0] + p[1] * o[3] + p[2] * o[6];
+  const bool ok = p[0] > 0.0 && o[8] > 0.0 && det > 0.0 && isfinite(det);
+  const double inv = 1.0 / det;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) o[k] *= inv;
+  return ok;
+}
+
 // Gauss-Jordan inversion of one SPD principal block per CTA, matrix in
-// registers: thread (ty, tx) owns rows ty + 16 ii and columns tx + 16 jj
-// (ii, jj < T), padding (index >= dim) is the identity.  Step k broadcasts
-// pivot row and column through shared memory (double-buffered: one barrier
-// per step).  Blocks with a non-positive pivot or a failed condition
-// certificate go to the fallback list.
-template <int T>
-__global__ void __launch_bounds__(256, 2) k_schwarz_gj(
-    int nsub, const int* __restrict__ sub_off, const int* __restrict__ sub_nodes,
-    const long long* __restrict__ gmap_off, const int* __restrict__ gmap, const int* __restrict__ adj_off, const long long* __restrict__ jbase,
-    const double* __restrict__ J, const long long* __restrict__ stage_off, double* __restrict__ stage,
+// registers: thread (ty, tx) of NT x NT owns the 9 x 9 tile at (9 ty, 9 tx),
+// padding (index >= dim) is the identity.  A step eliminates the three
+// unknowns of a node: its rows and columns are published in shared memory (R
+// with the identity, C with minus the identity in the pivot's place, the
+// owners' own copies cleared), P^-1 R is formed once, and a_ij - C_i (P^-1 R)_j
+// is the Gauss-Jordan step everywhere: row block, column block, pivot and the
+// rank-3 update.  Blocks with a non-positive pivot or a failed condition
+// certificate go to the fallback list; the others are stored symmetrized.
+// 27 steps of two barriers instead of 81 of one, and a tile of three nodes makes
+// the pivot's place in it a compile-time one and 243 FMAs follow 54 loads: 1,728
+// blocks of 81 x 81 in 303 us (16 x 16 threads with 6 x 6 entries each, scalar
+// steps: 432 us and 44 us for the symmetrization; with node steps 483).  Bound
+// by latency: 244 registers leave two CTAs of three warps per SM, and three
+// spill (765 us).
+template <int NT>
+__global__ void __launch_bounds__((NT * NT + 31) / 32 * 32) k_schwarz_gj(
+    const int* __restrict__ sub_off, const int* __restrict__ sub_nodes, const long long* __restrict__ gmap_off,
+    const int* __restrict__ gmap, const int* __restrict__ adj_off, const long long* __restrict__ jbase,
+    const double* __restrict__ J, const long long* __restrict__ stage_off, double* __restrict__ sym,
     int* __restrict__ fallback) {
-  constexpr int M = 16 * T;
-  __shared__ double s_row[2][M], s_col[2][M], s_piv[2];
-  __shared__ int s_g[27], s_rl[27];
+  constexpr int M = 9 * NT, TPB = (NT * NT + 31) / 32 * 32;
+  extern __shared__ double s_mat[];  // the inverse, dim x (dim | 1), for the symmetrization
+  __shared__ double s_r[2][3][M], s_c[2][3][M], s_p[2][9], s_t[2][3][M];
+  __shared__ int s_rl[27];
   __shared__ long long s_jb[27];
   __shared__ double s_red;
+  __shared__ int s_ok;
   const int sidx = blockIdx.x;
   const int n = sub_off[sidx + 1] - sub_off[sidx];
   const int dim = 3 * n;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int tx = threadIdx.x % NT, ty = threadIdx.x / NT;
+  const bool on = threadIdx.x < NT * NT;
   const int* nodes = sub_nodes + sub_off[sidx];
   if (threadIdx.x < n) {
-    int g = nodes[threadIdx.x];
-    s_g[threadIdx.x] = g;
+    const int g = nodes[threadIdx.x];
     s_rl[threadIdx.x] = 3 * (adj_off[g + 1] - adj_off[g]);
     s_jb[threadIdx.x] = jbase[g];
   }
   __syncthreads();
+  // gather the principal block, one node pair per thread at a time, then every
+  // thread takes its tile
   const int* gm = gmap + gmap_off[sidx];
-  double a[T][T];
-  double fa = 0.0;
+  double v1[1] = {0.0};
+#pragma unroll 4
+  for (int k = threadIdx.x; k < n * n; k += TPB) {
+    const int I = k / n, Jn = k - I * n;
+    const double* src = J + s_jb[I] + gm[k];
+    const int rl = s_rl[I];
+    double v[9];
 #pragma unroll
-  for (int ii = 0; ii < T; ++ii) {
-    const int r = ty + 16 * ii;
+    for (int q = 0; q < 9; ++q) v[q] = __ldg(src + (q / 3) * rl + q % 3);
 #pragma unroll
-    for (int jj = 0; jj < T; ++jj) {
-      const int c = tx + 16 * jj;
-      double v = (r == c) ? 1.0 : 0.0;
-      if (r < dim && c < dim) {
-        const int I = r / 3, i = r - 3 * I, Jn = c / 3, j = c - 3 * Jn;
-        v = J[s_jb[I] + gm[I * n + Jn] + i * s_rl[I] + j];
-        fa += v * v;
-      }
-      a[ii][jj] = v;
+    for (int q = 0; q < 9; ++q) {
+      v1[0] += v[q] * v[q];
+      s_mat[(3 * I + q / 3) * (dim | 1) + 3 * Jn + q % 3] = v[q];
     }
   }
-  double v1[1] = {fa};
-  block_sum<1>(v1);
+  block_sum<1>(v1);  // (and every entry is in place)
   if (threadIdx.x == 0) s_red = sqrt(v1[0]);
+  double a[9][9];
+#pragma unroll
+  for (int ii = 0; ii < 9; ++ii)
+#pragma unroll
+    for (int jj = 0; jj < 9; ++jj) {
+      const int r = 9 * ty + ii, c = 9 * tx + jj;
+      a[ii][jj] = on && r < dim && c < dim ? s_mat[r * (dim | 1) + c] : (r == c ? 1.0 : 0.0);
+    }
   bool ok = true;
-  // Step k: the owners of pivot row and column publish them (the pivot
-  // itself separately; in its place 1 in the row and -1 in the column) and
-  // zero their copies, so that one FMA a_ij - c_i r_j / piv per entry gives the
-  // Gauss-Jordan step everywhere: row k -> r_j / piv, column k -> -c_i / piv,
-  // pivot -> 1 / piv, the rest the rank-1 update.
-  for (int k = 0; k < dim; ++k) {
-    const int buf = k & 1;
-    const int kq = k >> 4, kr = k & 15;
-    if (ty == kr) {
+  int buf = 0;
+#pragma unroll 1
+  for (int b = 0; b < NT && ok; ++b) {
 #pragma unroll
-      for (int ii = 0; ii < T; ++ii)
-        if (ii == kq) {
+    for (int q = 0; q < 3; ++q) {
+      if (9 * b + 3 * q < dim && ok) {
+        // rows first: publishing the columns clears entries of the pivot block
+        if (on && ty == b) {
 #pragma unroll
-          for (int jj = 0; jj < T; ++jj) {
-            const bool pk = (tx == kr) && (jj == kq);
-            s_row[buf][tx + 16 * jj] = pk ? 1.0 : a[ii][jj];
-            if (pk) s_piv[buf] = a[ii][jj];
-            a[ii][jj] = 0.0;
-          }
+          for (int d = 0; d < 3; ++d)
+#pragma unroll
+            for (int jj = 0; jj < 9; ++jj) {
+              const bool pk = tx == b && jj / 3 == q;
+              s_r[buf][d][9 * tx + jj] = pk ? (jj - 3 * q == d ? 1.0 : 0.0) : a[3 * q + d][jj];
+              if (pk) s_p[buf][3 * d + jj - 3 * q] = a[3 * q + d][jj];
+              a[3 * q + d][jj] = 0.0;
+            }
         }
-    }
-    if (tx == kr) {
+        if (on && tx == b) {
 #pragma unroll
-      for (int jj = 0; jj < T; ++jj)
-        if (jj == kq) {
+          for (int d = 0; d < 3; ++d)
 #pragma unroll
-          for (int ii = 0; ii < T; ++ii) {
-            s_col[buf][ty + 16 * ii] = ((ty == kr) && (ii == kq)) ? -1.0 : a[ii][jj];
-            a[ii][jj] = 0.0;
-          }
+            for (int ii = 0; ii < 9; ++ii) {
+              const bool pk = ty == b && ii / 3 == q;
+              s_c[buf][d][9 * ty + ii] = pk ? (ii - 3 * q == d ? -1.0 : 0.0) : a[ii][3 * q + d];
+              a[ii][3 * q + d] = 0.0;
+            }
         }
+        __syncthreads();
+        double pi[9];
+        ok = inv3_spd(s_p[buf], pi);  // the same in every thread
+        if (ok) {
+          for (int j = threadIdx.x; j < M; j += TPB) {
+            const double r0 = s_r[buf][0][j], r1 = s_r[buf][1][j], r2 = s_r[buf][2][j];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) s_t[buf][d][j] = pi[3 * d] * r0 + pi[3 * d + 1] * r1 + pi[3 * d + 2] * r2;
+          }
+          __syncthreads();
+          if (on) {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+              double rj[9];
+#pragma unroll
+              for (int jj = 0; jj < 9; ++jj) rj[jj] = s_t[buf][d][9 * tx + jj];
+#pragma unroll
+              for (int ii = 0; ii < 9; ++ii) {
+                const double ci = s_c[buf][d][9 * ty + ii];
+#pragma unroll
+                for (int jj = 0; jj < 9; ++jj) a[ii][jj] = __fma_rn(-ci, rj[jj], a[ii][jj]);
+              }
+            }
+          }
+          buf ^= 1;
+        }
+      }
     }
-    __syncthreads();
-    const double piv = s_piv[buf];
-    if (!(piv > 0.0) || !isfinite(piv)) {
-      ok = false;
-      break;
-    }
-    const double inv = 1.0 / piv;
-    double rj[T], ci[T];
-#pragma unroll
-    for (int jj = 0; jj < T; ++jj) rj[jj] = s_row[buf][tx + 16 * jj] * inv;
-#pragma unroll
-    for (int ii = 0; ii < T; ++ii) ci[ii] = s_col[buf][ty + 16 * ii];
-#pragma unroll
-    for (int ii = 0; ii < T; ++ii)
-#pragma unroll
-      for (int jj = 0; jj < T; ++jj) a[ii][jj] = __fma_rn(-ci[ii], rj[jj], a[ii][jj]);
   }
-  double fi = 0.0;
-  if (ok) {
+  double v2[1] = {0.0};
+  if (ok && on) {
 #pragma unroll
-    for (int ii = 0; ii < T; ++ii)
+    for (int ii = 0; ii < 9; ++ii)
 #pragma unroll
-      for (int jj = 0; jj < T; ++jj) {
-        const int r = ty + 16 * ii, c = tx + 16 * jj;
-        if (r < dim && c < dim) fi += a[ii][jj] * a[ii][jj];
+      for (int jj = 0; jj < 9; ++jj) {
+        const int r = 9 * ty + ii, c = 9 * tx + jj;
+        if (r < dim && c < dim) {
+          v2[0] += a[ii][jj] * a[ii][jj];
+          s_mat[r * (dim | 1) + c] = a[ii][jj];
+        }
       }
   }
-  double v2[1] = {fi};
   block_sum<1>(v2);  // uniform: `ok` is the same in every thread
-  __shared__ int s_ok;
   if (threadIdx.x == 0) {
     const double cond = s_red * sqrt(v2[0]);
     s_ok = ok && (cond <= 1e12) && isfinite(cond);
@@ -188,21 +237,20 @@ __global__ void __launch_bounds__(256, 2) k_schwarz_gj(
   }
   __syncthreads();
   if (!s_ok) return;
-  double* out = stage + stage_off[sidx];
-#pragma unroll
-  for (int ii = 0; ii < T; ++ii)
-#pragma unroll
-    for (int jj = 0; jj < T; ++jj) {
-      const int r = ty + 16 * ii, c = tx + 16 * jj;
-      if (r < dim && c < dim) out[r * dim + c] = a[ii][jj];
-    }
+  // symmetric part (the elimination is symmetric only up to rounding)
+  double* out = sym + stage_off[sidx];
+  for (int k = threadIdx.x; k < dim * dim; k += TPB) {
+    const int r = k / dim, c = k - r * dim;
+    out[k] = 0.5 * (s_mat[r * (dim | 1) + c] + s_mat[c * (dim | 1) + r]);
+  }
 }
 
 // Eigen path for the blocks listed by k_schwarz_gj (count in fallback[0]).
 __global__ void __launch_bounds__(FACTOR_TPB) k_schwarz_factor(
     const int* __restrict__ fallback, const int* __restrict__ sub_off, const int* __restrict__ sub_nodes,
     const long long* __restrict__ gmap_off, const int* __restrict__ gmap, const int* __restrict__ adj_off, const long long* __restrict__ jbase,
-    const double* __restrict__ J, const long long* __restrict__ stage_off, double* __restrict__ stage, int* err) {
+    const double* __restrict__ J, const long long* __restrict__ stage_off, double* __restrict__ stage,
+    double* __restrict__ sym, int* err) {
   if ((int)blockIdx.x >= fallback[0]) return;
   extern __shared__ double smem[];
   const int sidx = fallback[1 + blockIdx.x];
@@ -273,6 +321,11 @@ __global__ void __launch_bounds__(FACTOR_TPB) k_schwarz_factor(
     for (int t = 0; t < dim; ++t) s += V[i * m + t] * A[t * m + t] * V[j * m + t];
     out[k] = s;
   }
+  __syncthreads();  // the block's own writes
+  for (int k = threadIdx.x; k < dim * dim; k += blockDim.x) {
+    const int r = k / dim, c = k % dim;
+    sym[stage_off[sidx] + k] = 0.5 * (out[k] + out[c * dim + r]);
+  }
 }
 
 __global__ void __launch_bounds__(256) k_schwarz_scatter(const int* __restrict__ subs, int count,
@@ -281,37 +334,19 @@ __global__ void __launch_bounds__(256) k_schwarz_scatter(const int* __restrict__
                                                          const long long* __restrict__ gmap_off,
                                                          const int* __restrict__ smap, const int* __restrict__ padj_off,
                                                          const long long* __restrict__ stage_off,
-                                                         const double* __restrict__ stage, double* __restrict__ pv) {
+                                                         const double* __restrict__ sym, double* __restrict__ pv) {
   const int sidx = subs[blockIdx.x];
   const int n = sub_off[sidx + 1] - sub_off[sidx];
   const int dim = 3 * n;
   const int* nodes = sub_nodes + sub_off[sidx];
   const int* sm = smap + gmap_off[sidx];
-  const double* blk = stage + stage_off[sidx];
-  // symmetric part of the staged block (the Gauss-Jordan inverse is symmetric
-  // only up to rounding; the eigen path's recomposition is symmetric exactly)
+  const double* blk = sym + stage_off[sidx];
   for (int k = threadIdx.x; k < dim * dim; k += blockDim.x) {
     int r = k / dim, c = k % dim;
     int I = r / 3, i = r % 3, Jn = c / 3, j = c % 3;
     int g = nodes[I];
     int rl = 3 * (padj_off[g + 1] - padj_off[g]);
-    pv[sm[I * n + Jn] + i * rl + j] += 0.5 * (blk[k] + blk[c * dim + r]);
-  }
-}
-
-// Symmetric part of every staged block (what the scatter adds), kept for the
-// block apply.
-__global__ void __launch_bounds__(256) k_schwarz_symmetrize(const int* __restrict__ sub_off,
-                                                            const long long* __restrict__ stage_off,
-                                                            const double* __restrict__ stage,
-                                                            double* __restrict__ sym) {
-  const int s = blockIdx.x;
-  const int dim = 3 * (sub_off[s + 1] - sub_off[s]);
-  const double* blk = stage + stage_off[s];
-  double* out = sym + stage_off[s];
-  for (int k = threadIdx.x; k < dim * dim; k += blockDim.x) {
-    const int r = k / dim, c = k % dim;
-    out[k] = 0.5 * (blk[k] + blk[c * dim + r]);
+    pv[sm[I * n + Jn] + i * rl + j] += blk[k];
   }
 }
 
@@ -528,7 +563,7 @@ static void check_err(DBuf<int>& e, cudaStream_t s) {
   }
 }
 
-// Adds the symmetric part of every staged block into the assembled values
+// Adds every symmetrized block into the assembled values
 // (one launch per Schwarz color: no two blocks of a color share a node).
 static void scatter_blocks(Precond& p, cudaStream_t s) {
   const int nc = (int)p.color_off.size() - 1;
@@ -537,7 +572,7 @@ static void scatter_blocks(Precond& p, cudaStream_t s) {
     if (cnt)
       (note_launch(), k_schwarz_scatter<<<cnt, 256, 0, s>>>(p.d_color_subs.p + b, cnt, p.d_sub_off.p, p.d_sub_nodes.p,
                                                              p.d_gmap_off.p, p.d_smap.p, p.d_adj_off.p, p.d_stage_off.p,
-                                                             p.staging.p, p.vals.p));
+                                                             p.bsym.p, p.vals.p));
   }
 }
 
@@ -559,24 +594,26 @@ void precond_update(Precond& p, const double* J, cudaStream_t s) {
   if (p.nsub > 0) {
     HOEFEM_CUDA(cudaMemsetAsync(p.d_fallback.p, 0, sizeof(int), s));
     const int dmax = 3 * p.max_nodes;
-#define HOEFEM_GJ(TT)                                                                                               \
-  (note_launch(), k_schwarz_gj<TT><<<(int)p.nsub, 256, 0, s>>>((int)p.nsub, p.d_sub_off.p, p.d_sub_nodes.p,         \
-                                                               p.d_gmap_off.p, p.d_gmap.p, m.d_adj_off.p, m.d_base.p, J,\
-                                                               p.d_stage_off.p, p.staging.p, p.d_fallback.p))
-    if (dmax <= 32) HOEFEM_GJ(2);
-    else if (dmax <= 48) HOEFEM_GJ(3);
-    else if (dmax <= 64) HOEFEM_GJ(4);
-    else HOEFEM_GJ(6);
+    const size_t gj_smem = sizeof(double) * (size_t)dmax * (dmax | 1);
+#define HOEFEM_GJ(NT)                                                                                                  \
+  do {                                                                                                                 \
+    HOEFEM_CUDA(cudaFuncSetAttribute(k_schwarz_gj<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gj_smem));    \
+    (note_launch(), k_schwarz_gj<NT><<<(int)p.nsub, (NT * NT + 31) / 32 * 32, gj_smem, s>>>(                           \
+                        p.d_sub_off.p, p.d_sub_nodes.p, p.d_gmap_off.p, p.d_gmap.p, m.d_adj_off.p, m.d_base.p, J,      \
+                        p.d_stage_off.p, p.bsym.p, p.d_fallback.p));                                                   \
+  } while (0)
+    // tiles of three nodes: subdomains of up to 9, 18 or 27 (the most) nodes
+    if (p.max_nodes <= 9) HOEFEM_GJ(3);
+    else if (p.max_nodes <= 18) HOEFEM_GJ(6);
+    else HOEFEM_GJ(9);
 #undef HOEFEM_GJ
     int m_max = (dmax + 1) & ~1;
     size_t smem = (size_t)(2 * m_max * m_max + m_max) * sizeof(double);
     (note_launch(), k_schwarz_factor<<<(int)p.nsub, FACTOR_TPB, smem, s>>>(p.d_fallback.p, p.d_sub_off.p,
                                                                            p.d_sub_nodes.p, p.d_gmap_off.p, p.d_gmap.p,
                                                                            m.d_adj_off.p, m.d_base.p, J, p.d_stage_off.p,
-                                                                           p.staging.p, p.d_err.p));
+                                                                           p.staging.p, p.bsym.p, p.d_err.p));
     HOEFEM_CUDA(cudaGetLastError());
-    (note_launch(), k_schwarz_symmetrize<<<(int)p.nsub, 256, 0, s>>>(p.d_sub_off.p, p.d_stage_off.p, p.staging.p,
-                                                                      p.bsym.p));
     if (!lazy) scatter_blocks(p, s);
   }
   if (!p.untreated.empty())
@@ -612,11 +649,59 @@ void precond_to_fp32(Precond& p, cudaStream_t s) {
   }
 }
 
+namespace {
+
+// z = P r from the symmetrized blocks: y_s = B_s r_s (thread j: column j = row
+// j, rows read by consecutive threads), then per DOF the sum over its
+// subdomains in ascending order, or the diagonal entry of an untreated node.
+__global__ void __launch_bounds__(96) k_apply_blocks(const int* __restrict__ sub_off, const int* __restrict__ sub_nodes,
+                                                     const long long* __restrict__ stage_off,
+                                                     const double* __restrict__ B, const int* __restrict__ slot,
+                                                     const double* __restrict__ r, double* __restrict__ y) {
+  __shared__ double rs[96];
+  const int o = sub_off[blockIdx.x], dim = 3 * (sub_off[blockIdx.x + 1] - o), j = threadIdx.x;
+  if (j < dim) rs[j] = r[3 * sub_nodes[o + j / 3] + j % 3];
+  __syncthreads();
+  if (j >= dim) return;
+  const double* Bj = B + stage_off[blockIdx.x] + j;
+  double acc = 0.0;
+#pragma unroll 27
+  for (int i = 0; i < dim; ++i) acc += Bj[(size_t)i * dim] * rs[i];
+  y[3 * slot[o + j / 3] + j % 3] = acc;
+}
+
+__global__ void __launch_bounds__(256) k_apply_gather(int n, const int* __restrict__ pair_off,
+                                                      const double* __restrict__ y,
+                                                      const unsigned char* __restrict__ diag_only,
+                                                      const long long* __restrict__ pbase,
+                                                      const double* __restrict__ pv, const double* __restrict__ r,
+                                                      double* __restrict__ z) {
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    const int a = t / 3, i = t - 3 * a;
+    double v = 0.0;
+    if (diag_only[a]) v = pv[pbase[a] + i] * r[t];
+    else
+      for (int q = pair_off[a]; q < pair_off[a + 1]; ++q) v += y[3 * q + i];
+    z[t] = v;
+  }
+}
+
+}  // namespace
+
 void precond_apply(const Precond& p, const double* r, double* z, cudaStream_t s) {
   HOEFEM_REQUIRE(p.ready, HOEFEM_ERR_INVALID_ARGUMENT, "preconditioner has not been updated");
   if (p.kind == PREC_DIAGONAL) {
     int n = (int)p.m->ndof;
     (note_launch(), k_mul<<<reduce_blocks_for(n), 256, 0, s>>>(n, p.diag.p, r, z));
+  } else if (p.block_apply && p.nsub > 0 && !p.vals_complete) {
+    // from the blocks: assembling the values first (one scatter per Schwarz
+    // color) costs more than the product.  Values that are assembled already,
+    // because something has read them, are applied as a matrix.
+    const int n = (int)p.m->ndof;
+    (note_launch(), k_apply_blocks<<<(int)p.nsub, 96, 0, s>>>(p.d_sub_off.p, p.d_sub_nodes.p, p.d_stage_off.p, p.bsym.p,
+                                                              p.d_npair.p, r, p.ysub.p));
+    (note_launch(), k_apply_gather<<<reduce_blocks_for(n), 256, 0, s>>>(n, p.d_npair_off.p, p.ysub.p, p.d_diag_only.p,
+                                                                        p.d_base.p, p.vals.p, r, z));
   } else {
     precond_assemble(p, s);
     NodeRows PR = p.rows();

@@ -35,7 +35,7 @@ struct Precond {
   DBuf<int> d_adj_off, d_adj, d_diag_slot, d_sub_off, d_sub_nodes, d_gmap, d_smap, d_color_subs, d_untreated;
   DBuf<long long> d_base, d_gmap_off;
   DBuf<unsigned char> d_diag_only;
-  DBuf<double> vals, staging;
+  DBuf<double> vals, staging;  // staging: the fallback's recomposed blocks
   DBuf<float> vals32;  // FP32 copy of the Schwarz values (mixed-precision apply)
   bool want_fp32 = false;
   DBuf<long long> d_stage_off;
@@ -52,6 +52,7 @@ struct Precond {
   // layout) applied as dense products into ysub (3 entries per subdomain
   // node), then summed per node over its subdomains in subdomain order.
   bool block_apply = true;
+  bool apply_pinned = false;  // the apply was chosen by the caller (hoefem_precond_set_block_apply)
   // With the block apply the CG reads the symmetrized blocks and, from the
   // assembled values, only the untreated (diagonal-only) entries, which every
   // update writes; the subdomain entries are scattered into the values when

@@ -355,7 +355,7 @@ int hoefem_integrator_set_precision(hoefem_integrator it, int precision, double 
    is one host loop).  Two engines run the same recurrence: the chunked engine
    on the CSR values in place (one cooperative launch per residual
    replacement; CUDA graphs of kernel chunks where that launch does not apply:
-   pinned SpMV variants, Schwarz as an assembled matrix, values not aligned to
+   pinned SpMV variants or a pinned Schwarz apply, values not aligned to
    16 bytes, nodes with more than 340 FP64 or 680 FP32 neighbours), and the
    persistent streamed CG (one cooperative launch per solve, the operator and
    the Schwarz blocks packed into stream layouts; for no preconditioner,
