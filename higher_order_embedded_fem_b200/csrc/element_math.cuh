@@ -124,6 +124,92 @@ __device__ __forceinline__ void tet4_jacobian(const R* Xc, R* J) {
     for (int j = 0; j < 3; ++j) J[3 * i + j] = -R(0.5) * Xc[i] + R(0.5) * Xc[3 * (j + 1) + i];
 }
 
+// ---- Hex27 in axis order -----------------------------------------------------
+// Node of place i + 3 j + 9 k, coordinate -1, 0, 1 for i, j, k = 0, 1, 2.
+__device__ const unsigned char g_hex27_at[27] = {0, 8,  1, 9, 20, 11, 3, 13, 2, 10, 21, 12, 22, 26,
+                                                 23, 15, 24, 14, 4, 16, 5, 17, 25, 18, 7, 19, 6};
+__device__ __forceinline__ int hex27_at(int place) { return g_hex27_at[place]; }
+
+// The one-dimensional quadratic functions p[3 axis + i] and their derivatives.
+__device__ __forceinline__ void hex27_axes(const double* xi, double* p, double* d) {
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const double x = xi[a], h = 0.5 * x;
+    p[3 * a] = h * x - h;
+    p[3 * a + 1] = 1.0 - x * x;
+    p[3 * a + 2] = h * x + h;
+    d[3 * a] = x - 0.5;
+    d[3 * a + 1] = -2.0 * x;
+    d[3 * a + 2] = x + 0.5;
+  }
+}
+// H[3 c + m] = sum over the nodes of v_c dN/dxi_m, summed axis by axis.  v: nine
+// rows (j + 3 k) of ten doubles, 3 i + c, 16-byte aligned.
+__device__ __forceinline__ void hex27_gradient(const double* v, const double* p, const double* d, double* H) {
+#pragma unroll
+  for (int n = 0; n < 9; ++n) H[n] = 0.0;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    double A[3] = {0, 0, 0}, B[3] = {0, 0, 0}, C[3] = {0, 0, 0};
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const double2* r = reinterpret_cast<const double2*>(v + 10 * (j + 3 * k));
+      double w[10];
+#pragma unroll
+      for (int n = 0; n < 5; ++n) {
+        const double2 t = r[n];
+        w[2 * n] = t.x;
+        w[2 * n + 1] = t.y;
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const double s = p[0] * w[c] + p[1] * w[3 + c] + p[2] * w[6 + c];
+        const double t = d[0] * w[c] + d[1] * w[3 + c] + d[2] * w[6 + c];
+        A[c] += p[3 + j] * t;
+        B[c] += d[3 + j] * s;
+        C[c] += p[3 + j] * s;
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      H[3 * c] += p[6 + k] * A[c];
+      H[3 * c + 1] += p[6 + k] * B[c];
+      H[3 * c + 2] += d[6 + k] * C[c];
+    }
+  }
+}
+// Value t of the 36 half edge vectors (3 (4 axis + edge) + component) of a Hex8
+// with its corners in axis order (x + 2 y + 4 z).
+__device__ __forceinline__ double hex8_edge(const double* corner, int t) {
+  const int axis = t / 12, ed = t / 3 % 4, c = t % 3;
+  const int lo = axis == 0 ? 2 * ed : (axis == 1 ? (ed & 1) | (ed & 2) << 1 : ed);
+  return 0.5 * (corner[3 * (lo + (1 << axis)) + c] - corner[3 * lo + c]);
+}
+// Jacobian of the trilinear geometry from them (16-byte aligned).
+__device__ __forceinline__ void hex8_jacobian_edges(const double* se, const double* xi, double* J) {
+  double lo[3], hi[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    lo[a] = 0.5 - 0.5 * xi[a];
+    hi[a] = 0.5 + 0.5 * xi[a];
+  }
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const int b = a == 0 ? 1 : 0, c = a == 2 ? 1 : 2;
+    const double w[4] = {lo[b] * lo[c], hi[b] * lo[c], lo[b] * hi[c], hi[b] * hi[c]};
+    double v[12];
+    const double2* r = reinterpret_cast<const double2*>(se + 12 * a);
+#pragma unroll
+    for (int n = 0; n < 6; ++n) {
+      const double2 t = r[n];
+      v[2 * n] = t.x;
+      v[2 * n + 1] = t.y;
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) J[3 * i + a] = w[0] * v[i] + w[1] * v[3 + i] + w[2] * v[6 + i] + w[3] * v[9 + i];
+  }
+}
+
 template <class R>
 __device__ __forceinline__ R det3(const R* m) {
   return m[0] * (m[4] * m[8] - m[7] * m[5]) - m[1] * (m[3] * m[8] - m[6] * m[5]) + m[2] * (m[3] * m[7] - m[6] * m[4]);
@@ -142,6 +228,20 @@ __device__ __forceinline__ R inv3(const R* m, R* o) {
   o[7] = -(m[0] * m[7] - m[6] * m[1]) / d;
   o[8] = (m[0] * m[4] - m[3] * m[1]) / d;
   return d;
+}
+
+// Cofactor matrix of m (= det m * m^-T) and det m, without divisions.
+__device__ __forceinline__ double cofactors(const double* m, double* c) {
+  c[0] = m[4] * m[8] - m[5] * m[7];
+  c[1] = m[5] * m[6] - m[3] * m[8];
+  c[2] = m[3] * m[7] - m[4] * m[6];
+  c[3] = m[2] * m[7] - m[1] * m[8];
+  c[4] = m[0] * m[8] - m[2] * m[6];
+  c[5] = m[1] * m[6] - m[0] * m[7];
+  c[6] = m[1] * m[5] - m[2] * m[4];
+  c[7] = m[2] * m[3] - m[0] * m[5];
+  c[8] = m[0] * m[4] - m[1] * m[3];
+  return m[0] * c[0] + m[1] * c[1] + m[2] * c[2];
 }
 
 // ---- materials (materials.rs) -----------------------------------------------
@@ -247,6 +347,110 @@ __device__ __forceinline__ void qp_pair_from(int kind, const QpState<R>& q, QpPa
   o.s2 = q.s2;
   o.s3 = q.s3;
   o.s4 = q.s4;
+}
+
+// What the pair contraction needs of a point (material_state of
+// element_math.cuh without the stress): the stable Neo-Hookean Cof F comes from
+// the minors instead of det F * F^-T, which takes nine FP64 divisions.
+// Returns false where F is doubtful (below).
+__device__ __forceinline__ bool det_doubtful(double det, const double* cof, double scale);
+__device__ __forceinline__ bool point_state(int kind, const double* F, double mu0, double lam0, QpPair<double>& o,
+                                            double* M1) {
+  if (kind == HOEFEM_MAT_SNH) {
+    const double mu = 4.0 / 3.0 * mu0, lam = lam0 + (1.0 - 2.0 / 12.0) * mu0;
+    const double alpha = 1.0 + mu / lam * 0.75;
+    double IC = 0.0;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      IC += F[k] * F[k];
+      o.T[k] = F[k];
+    }
+    const double J = cofactors(F, M1);
+    const double ib = 1.0 / (IC + 1.0);
+    o.s1 = mu * (1.0 - ib);
+    o.s2 = mu * 2.0 * ib * ib;
+    o.s3 = lam * (J - alpha);
+    o.s4 = lam;
+    return !det_doubtful(J, M1, 1.0);
+  }
+  QpState<double> st;
+  stvk_state(F, mu0, lam0, st, false);
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    o.T[k] = st.M2[k];
+    M1[k] = st.M1[k];
+  }
+  o.s1 = st.s1;
+  o.s4 = st.s4;
+  o.s2 = o.s3 = 0.0;
+  return true;
+}
+
+// ---- singular points ---------------------------------------------------------
+// A point is singular when the determinant of its Jacobian, or of F for the
+// stable Neo-Hookean material, is exactly zero in the node sums of the colored
+// kernels.  The faster kernels form both in another order, so a determinant that
+// is zero there may be a rounding residue here: they ask whether it is zero to
+// rounding (det_doubtful, m of order scale), and only such points are evaluated
+// again as those sums (tet10_singular, hex27_singular).
+__device__ __forceinline__ bool det_doubtful(double det, const double* cof, double scale) {
+  double s = 0.0;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) s += fabs(cof[k]);
+  return !(fabs(det) > 1e-10 * s * scale);
+}
+// corner: 4 x 3, un: 10 x 3.
+__device__ __noinline__ bool tet10_singular(int kind, const double* corner, const double* un, const double* point) {
+  const double xi[3] = {point[0], point[1], point[2]};
+  double J[9], Ji[9], F[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  tet4_jacobian(corner, J);
+  if (inv3(J, Ji) == 0.0) return true;
+  if (kind != HOEFEM_MAT_SNH) return false;
+#pragma unroll 1
+  for (int I = 0; I < 10; ++I) {
+    double gr[3], G[3];
+    tet10_grad(I, xi, gr);
+    for (int k = 0; k < 3; ++k) G[k] = Ji[k] * gr[0] + Ji[3 + k] * gr[1] + Ji[6 + k] * gr[2];
+    for (int c = 0; c < 3; ++c)
+      for (int k = 0; k < 3; ++k) F[3 * c + k] += un[3 * I + c] * G[k];
+  }
+  F[0] += 1.0;
+  F[4] += 1.0;
+  F[8] += 1.0;
+  return det3(F) == 0.0;
+}
+// corner: 8 x 3 and un (nine rows of ten), both in axis order.
+__device__ __noinline__ bool hex27_singular(int kind, const double* corner, const double* un, const double* point) {
+  const double xi[3] = {point[0], point[1], point[2]};
+  double Xc[24], J[9], Ji[9], F[9];
+#pragma unroll 1
+  for (int I = 0; I < 8; ++I) {
+    const signed char* a = c_hex27_alpha[I];
+    for (int k = 0; k < 3; ++k) Xc[3 * I + k] = corner[3 * ((a[0] > 0) + 2 * (a[1] > 0) + 4 * (a[2] > 0)) + k];
+  }
+  hex8_jacobian(Xc, xi, J);
+  if (inv3(J, Ji) == 0.0) return true;
+  if (kind != HOEFEM_MAT_SNH) return false;
+#pragma unroll 1
+  for (int n = 0; n < 9; ++n) {  // a warp's sum over its lanes, lane = node
+    const int c = n / 3, k = n - 3 * c;
+    double t[32];
+#pragma unroll 1
+    for (int I = 0; I < 32; ++I) {
+      t[I] = 0.0;
+      if (I >= 27) continue;
+      const signed char* a = c_hex27_alpha[I];
+      double gr[3];
+      hex27_grad(I, xi, gr);
+      const double G = Ji[k] * gr[0] + Ji[3 + k] * gr[1] + Ji[6 + k] * gr[2];
+      t[I] = __dmul_rn(un[10 * (a[1] + 1 + 3 * (a[2] + 1)) + 3 * (a[0] + 1) + c], G);
+    }
+#pragma unroll 1
+    for (int o = 16; o > 0; o >>= 1)
+      for (int I = 0; I < o; ++I) t[I] += t[I + o];
+    F[n] = t[0] + (c == k ? 1.0 : 0.0);
+  }
+  return det3(F) == 0.0;
 }
 
 // Stiffness block of node pair (I row, J column), added into acc (3x3 row-major).

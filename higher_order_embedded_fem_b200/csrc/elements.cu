@@ -1,14 +1,12 @@
-// Element kernels: hyperelastic internal force, tangent stiffness fused with
-// the colored CSR scatter, and the consistent mass matrix (FP64).
+// Element kernels: tangent stiffness fused with the colored CSR scatter, and
+// the consistent mass matrix (FP64); the internal forces are in forces.cu.
 //
 // Reference: fenris/src/assembly.rs:618-797 (element mass / elliptic term /
-// stiffness), :252-314 + :1042-1075 (colored CSR scatter), :915-966 (colored
-// force scatter); materials in fenris/src/solid/materials.rs.
+// stiffness), :252-314 + :1042-1075 (colored CSR scatter); materials in
+// fenris/src/solid/materials.rs.
 //
 // Layout: connectivity is SoA (conn[I * ne + e]) so that the lanes that own
-// the nodes of one element read it with one transaction per node.  Forces:
-// one warp per Tet10 element with a lane per quadrature point (affine
-// geometry), eight warps per Hex27 element over its points.  Stiffness: 64
+// the nodes of one element read it with one transaction per node.  Stiffness: 64
 // threads per Tet10 element (4 per CTA; the per-point phase one lane per
 // point), 384 per Hex27 element.  Per quadrature point the kernel builds the
 // per-node vectors a_I = sqrt(w |det J|) J^-T grad N_I, b_I = F a_I and
@@ -31,264 +29,6 @@ namespace {
 
 constexpr int TPB = 128;
 
-
-// ============================================================================
-// Internal force: warp per element (nodes <= 32), per-color launch.
-// f_e(:, I) += -(P J^-T grad N_I) w |det J|  (assembly.rs:695-708)
-// ============================================================================
-template <int NN>
-__global__ void __launch_bounds__(TPB) k_forces(const BlockDev b, const int* __restrict__ elems, int count,
-                                                const double* __restrict__ X, const double* __restrict__ u,
-                                                double* __restrict__ f, MatDev mat, int* err,
-                                                double* __restrict__ fst = nullptr) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int idx = blockIdx.x * (TPB / 32) + warp;
-  __shared__ double s_corner[TPB / 32][24];
-  if (idx >= count) return;
-  const int e = elems[idx];
-  if (b.scene_active && !b.scene_active[b.escene[e]]) return;
-  const bool own = lane < NN;
-  int g = own ? b.conn[lane * b.ne + e] : 0;
-  double Xl[3] = {0, 0, 0}, ul[3] = {0, 0, 0};
-  if (own) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) { Xl[k] = X[3 * g + k]; ul[k] = u[3 * g + k]; }
-  }
-  constexpr int NC = (NN == 10) ? 4 : 8;
-  if (lane < NC) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) s_corner[warp][3 * lane + k] = Xl[k];
-  }
-  __syncwarp();
-  double J[9], Ji[9], detJ = 0.0;
-  if (NN == 10) {
-    tet4_jacobian(s_corner[warp], J);
-    detJ = inv3(J, Ji);
-  }
-  double fl[3] = {0, 0, 0};
-  int q0, nq;
-  quad_rule(b, e, q0, nq);
-  bool ok = true;
-  for (int q = 0; q < nq; ++q) {
-    const double xi[3] = {b.qp[3 * (q0 + q)], b.qp[3 * (q0 + q) + 1], b.qp[3 * (q0 + q) + 2]};
-    const double w = b.qw[q0 + q];
-    if (NN == 27) {
-      hex8_jacobian(s_corner[warp], xi, J);
-      detJ = inv3(J, Ji);
-    }
-    if (detJ == 0.0) { ok = false; break; }
-    double gr[3] = {0, 0, 0}, G[3] = {0, 0, 0};
-    if (own) {
-      if (NN == 10) tet10_grad(lane, xi, gr); else hex27_grad(lane, xi, gr);
-      // G = J^-T gr
-#pragma unroll
-      for (int k = 0; k < 3; ++k) G[k] = Ji[k] * gr[0] + Ji[3 + k] * gr[1] + Ji[6 + k] * gr[2];
-    }
-    // F(c,k) = delta + sum_I u_I[c] G_I[k]
-    double F[9];
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-      for (int k = 0; k < 3; ++k) F[3 * c + k] = warp_sum(ul[c] * G[k]) + (c == k ? 1.0 : 0.0);
-    QpState<double> st;
-    const double emu = b.emat ? b.emat[2 * e] : mat.mu, elam = b.emat ? b.emat[2 * e + 1] : mat.lambda;
-    if (!material_state(mat.kind, F, emu, elam, st, true)) { ok = false; break; }
-    if (own) {
-      double sc = w * fabs(detJ);
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-        fl[i] += -(st.P[3 * i] * G[0] + st.P[3 * i + 1] * G[1] + st.P[3 * i + 2] * G[2]) * sc;
-    }
-  }
-  if (!ok) {
-    if (lane == 0) set_error(err, HOEFEM_ERR_SINGULAR);
-    return;
-  }
-  if (own) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      if (fst) fst[((size_t)e * NN + lane) * 3 + i] = fl[i];
-      else f[3 * g + i] += fl[i];
-    }
-  }
-}
-
-// ============================================================================
-// Internal force, Tet10 (affine geometry, uniform rule of <= 32 points): warp
-// per element, lane q evaluates quadrature point q (F from all 10 nodes, the
-// stress once) and writes its contribution to every node into shared memory;
-// the node lanes then add the points' contributions in point order, as the
-// sequential loop of the reference does.
-// ============================================================================
-constexpr int T10_FSTRIDE = 31;  // doubles per point row (30 used; odd stride)
-
-__global__ void __launch_bounds__(TPB) k_forces_tet10(const BlockDev b, const int* __restrict__ elems, int count,
-                                                      const double* __restrict__ X, const double* __restrict__ u,
-                                                      double* __restrict__ f, MatDev mat, int* err,
-                                                      double* __restrict__ fst = nullptr) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int idx = blockIdx.x * (TPB / 32) + warp;
-  __shared__ double s_corner[TPB / 32][12];
-  __shared__ double s_u[TPB / 32][30];
-  __shared__ double s_f[TPB / 32][32 * T10_FSTRIDE];
-  if (idx >= count) return;
-  const int e = elems[idx];
-  if (b.scene_active && !b.scene_active[b.escene[e]]) return;
-  int g = 0;
-  if (lane < 10) {
-    g = b.conn[lane * b.ne + e];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const double x = X[3 * g + k];
-      s_u[warp][3 * lane + k] = u[3 * g + k];
-      if (lane < 4) s_corner[warp][3 * lane + k] = x;
-    }
-  }
-  __syncwarp();
-  double J[9], Ji[9];
-  tet4_jacobian(s_corner[warp], J);
-  const double detJ = inv3(J, Ji);
-  const int nq = b.nq;
-  bool ok = detJ != 0.0;
-  if (ok && lane < nq) {
-    const double xi[3] = {b.qp[3 * lane], b.qp[3 * lane + 1], b.qp[3 * lane + 2]};
-    double F[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll
-    for (int I = 0; I < 10; ++I) {
-      double gr[3], G[3];
-      tet10_grad(I, xi, gr);
-#pragma unroll
-      for (int k = 0; k < 3; ++k) G[k] = Ji[k] * gr[0] + Ji[3 + k] * gr[1] + Ji[6 + k] * gr[2];
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) F[3 * c + k] += s_u[warp][3 * I + c] * G[k];
-    }
-    F[0] += 1.0;
-    F[4] += 1.0;
-    F[8] += 1.0;
-    QpState<double> st;
-    const double emu = b.emat ? b.emat[2 * e] : mat.mu, elam = b.emat ? b.emat[2 * e + 1] : mat.lambda;
-    ok = material_state(mat.kind, F, emu, elam, st, true);
-    if (ok) {
-      const double sc = b.qw[lane] * fabs(detJ);
-      double* out = s_f[warp] + lane * T10_FSTRIDE;
-#pragma unroll
-      for (int I = 0; I < 10; ++I) {
-        double gr[3], G[3];
-        tet10_grad(I, xi, gr);
-#pragma unroll
-        for (int k = 0; k < 3; ++k) G[k] = Ji[k] * gr[0] + Ji[3 + k] * gr[1] + Ji[6 + k] * gr[2];
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-          out[3 * I + i] = -(st.P[3 * i] * G[0] + st.P[3 * i + 1] * G[1] + st.P[3 * i + 2] * G[2]) * sc;
-      }
-    }
-  }
-  ok = __all_sync(0xffffffffu, ok);
-  __syncwarp();
-  if (!ok) {
-    if (lane == 0) set_error(err, HOEFEM_ERR_SINGULAR);
-    return;
-  }
-  if (lane < 10) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      double acc = 0.0;
-      for (int q = 0; q < nq; ++q) acc += s_f[warp][q * T10_FSTRIDE + 3 * lane + i];
-      if (fst) fst[((size_t)e * 10 + lane) * 3 + i] = acc;
-      else f[3 * g + i] += acc;
-    }
-  }
-}
-
-// ============================================================================
-// Internal force, Hex27: FW warps per element (one CTA), warp w takes the
-// quadrature points w, w + FW, ...; the per-warp node forces are summed in
-// shared memory in warp order (deterministic) and scattered once.  A color
-// of a few hundred elements then fills the GPU with FW times more warps.
-// ============================================================================
-constexpr int FW = 8;
-
-__global__ void __launch_bounds__(32 * FW, 2) k_forces_hex27(const BlockDev b, const int* __restrict__ elems, int count,
-                                                         const double* __restrict__ X, const double* __restrict__ u,
-                                                         double* __restrict__ f, MatDev mat, int* err,
-                                                         double* __restrict__ fst = nullptr) {
-  constexpr int NN = 27;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __shared__ double s_corner[24];
-  __shared__ double s_f[FW][NN][3];
-  __shared__ int s_ok;
-  const int e = elems[blockIdx.x];
-  if (b.scene_active && !b.scene_active[b.escene[e]]) return;  // uniform over the CTA
-  const bool own = lane < NN;
-  const int g = own ? b.conn[lane * b.ne + e] : 0;
-  double ul[3] = {0, 0, 0};
-  if (own) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) ul[k] = u[3 * g + k];
-    if (warp == 0 && lane < 8) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) s_corner[3 * lane + k] = X[3 * g + k];
-    }
-  }
-  if (threadIdx.x == 0) s_ok = 1;
-  __syncthreads();
-  int q0, nq;
-  quad_rule(b, e, q0, nq);
-  const double emu = b.emat ? b.emat[2 * e] : mat.mu, elam = b.emat ? b.emat[2 * e + 1] : mat.lambda;
-  double fl[3] = {0, 0, 0};
-  for (int q = warp; q < nq; q += FW) {
-    const double xi[3] = {b.qp[3 * (q0 + q)], b.qp[3 * (q0 + q) + 1], b.qp[3 * (q0 + q) + 2]};
-    const double w = b.qw[q0 + q];
-    double J[9], Ji[9];
-    hex8_jacobian(s_corner, xi, J);
-    const double detJ = inv3(J, Ji);
-    double gr[3] = {0, 0, 0}, G[3] = {0, 0, 0};
-    if (own) {
-      hex27_grad(lane, xi, gr);
-#pragma unroll
-      for (int k = 0; k < 3; ++k) G[k] = Ji[k] * gr[0] + Ji[3 + k] * gr[1] + Ji[6 + k] * gr[2];
-    }
-    double F[9];
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-      for (int k = 0; k < 3; ++k) F[3 * c + k] = warp_sum(ul[c] * G[k]) + (c == k ? 1.0 : 0.0);
-    QpState<double> st;
-    if (detJ == 0.0 || !material_state(mat.kind, F, emu, elam, st, true)) {
-      if (lane == 0) s_ok = 0;
-      break;
-    }
-    if (own) {
-      const double sc = w * fabs(detJ);
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-        fl[i] += -(st.P[3 * i] * G[0] + st.P[3 * i + 1] * G[1] + st.P[3 * i + 2] * G[2]) * sc;
-    }
-  }
-  if (own) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) s_f[warp][lane][i] = fl[i];
-  }
-  __syncthreads();
-  if (!s_ok) {
-    if (threadIdx.x == 0) set_error(err, HOEFEM_ERR_SINGULAR);
-    return;
-  }
-  if (threadIdx.x < 3 * NN) {
-    const int I = threadIdx.x / 3, i = threadIdx.x % 3;
-    double acc = 0.0;
-#pragma unroll
-    for (int w = 0; w < FW; ++w) acc += s_f[w][I][i];
-    if (fst) {
-      fst[((size_t)e * NN + I) * 3 + i] = acc;
-    } else {
-      const int gI = b.conn[I * b.ne + e];
-      f[3 * gI + i] += acc;
-    }
-  }
-}
 
 // ============================================================================
 // Stiffness + scatter.  TPE threads (TPE / 32 warps) own one element, EPC
@@ -637,43 +377,7 @@ void init_pairs() {
   g_pairs_ready = true;
 }
 
-template <class F>
-void for_each_color(const Block& blk, F&& fn) {
-  const int nc = (int)blk.color_off.size() - 1;
-  for (int c = 0; c < nc; ++c) {
-    int begin = (int)blk.color_off[c];
-    int cnt = (int)(blk.color_off[c + 1] - begin);
-    if (cnt > 0) fn(blk.d_color_elems.p + begin, cnt);
-  }
-}
-
 }  // namespace
-
-void launch_forces(const Model& m, const MatDev& mat, const double* u, double* f, cudaStream_t s) {
-  for (const Block* bp : m.blocks) {
-    BlockDev bd = bp->dev();
-    auto launch = [&](const int* elems, int cnt, double* fst) {
-      int grid = (cnt + TPB / 32 - 1) / (TPB / 32);
-      if (bp->kind == HOEFEM_ELEM_TET10 && bd.uniform && bd.nq <= 32)
-        (note_launch(), k_forces_tet10<<<grid, TPB, 0, s>>>(bd, elems, cnt, m.d_X.p, u, f, mat, m.d_err.p, fst));
-      else if (bp->kind == HOEFEM_ELEM_TET10)
-        (note_launch(), k_forces<10><<<grid, TPB, 0, s>>>(bd, elems, cnt, m.d_X.p, u, f, mat, m.d_err.p, fst));
-      else
-        (note_launch(), k_forces_hex27<<<cnt, 32 * FW, 0, s>>>(bd, elems, cnt, m.d_X.p, u, f, mat, m.d_err.p, fst));
-    };
-    if (stiffness_pairs_eligible(m, *bp)) {
-      // every element in one launch into per-element node forces, then the
-      // per-node gather (element order)
-      double* fst = forces_stage_buffer(m, *bp, s);
-      if (bp->ne > 0) launch(bp->d_color_elems.p, (int)bp->ne, fst);
-      HOEFEM_CUDA(cudaGetLastError());
-      forces_gather(m, *bp, f, s);
-    } else {
-      for_each_color(*bp, [&](const int* elems, int cnt) { launch(elems, cnt, nullptr); });
-    }
-  }
-  HOEFEM_CUDA(cudaGetLastError());
-}
 
 template <int NN, class R>
 void launch_stiffness_kind(const Model& m, const Block& blk, const MatDev& mat, const double* u, double* vals,

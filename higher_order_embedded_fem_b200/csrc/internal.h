@@ -199,6 +199,17 @@ struct MatDev {
   double mu, lambda;
 };
 
+// fn(elements, count) for each color of a block: no two elements of a color share a node.
+template <class F>
+void for_each_color(const Block& blk, F&& fn) {
+  const int nc = (int)blk.color_off.size() - 1;
+  for (int c = 0; c < nc; ++c) {
+    int begin = (int)blk.color_off[c];
+    int cnt = (int)(blk.color_off[c + 1] - begin);
+    if (cnt > 0) fn(blk.d_color_elems.p + begin, cnt);
+  }
+}
+
 // ---- element kernels (elements.cu) -----------------------------------------
 void launch_forces(const Model& m, const MatDev& mat, const double* u, double* f, cudaStream_t s);
 enum Precision { PRECISION_FP64 = 0, PRECISION_FP32 = 1 };

@@ -56,56 +56,6 @@ __host__ __device__ constexpr int sym4(int x, int y) { return x <= y ? 4 * x - x
 // above bit 12 (values are multiples of 1: 16 is stored as 7).
 __constant__ int c_terms[NPAIR][4];
 
-// Cofactor matrix of m (= det m * m^-T) and det m, without divisions.
-__device__ __forceinline__ double cofactors(const double* m, double* c) {
-  c[0] = m[4] * m[8] - m[5] * m[7];
-  c[1] = m[5] * m[6] - m[3] * m[8];
-  c[2] = m[3] * m[7] - m[4] * m[6];
-  c[3] = m[2] * m[7] - m[1] * m[8];
-  c[4] = m[0] * m[8] - m[2] * m[6];
-  c[5] = m[1] * m[6] - m[0] * m[7];
-  c[6] = m[1] * m[5] - m[2] * m[4];
-  c[7] = m[2] * m[3] - m[0] * m[5];
-  c[8] = m[0] * m[4] - m[1] * m[3];
-  return m[0] * c[0] + m[1] * c[1] + m[2] * c[2];
-}
-
-// What the pair contraction needs of a point (material_state of
-// element_math.cuh without the stress): the stable Neo-Hookean Cof F comes from
-// the minors instead of det F * F^-T, which takes nine FP64 divisions.
-__device__ __forceinline__ bool point_state(int kind, const double* F, double mu0, double lam0, QpPair<double>& o,
-                                            double* M1) {
-  if (kind == HOEFEM_MAT_SNH) {
-    const double mu = 4.0 / 3.0 * mu0, lam = lam0 + (1.0 - 2.0 / 12.0) * mu0;
-    const double alpha = 1.0 + mu / lam * 0.75;
-    double IC = 0.0;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) {
-      IC += F[k] * F[k];
-      o.T[k] = F[k];
-    }
-    const double J = cofactors(F, M1);
-    if (J == 0.0) return false;
-    const double ib = 1.0 / (IC + 1.0);
-    o.s1 = mu * (1.0 - ib);
-    o.s2 = mu * 2.0 * ib * ib;
-    o.s3 = lam * (J - alpha);
-    o.s4 = lam;
-    return true;
-  }
-  QpState<double> st;
-  stvk_state(F, mu0, lam0, st, false);
-#pragma unroll
-  for (int k = 0; k < 9; ++k) {
-    o.T[k] = st.M2[k];
-    M1[k] = st.M1[k];
-  }
-  o.s1 = st.s1;
-  o.s4 = st.s4;
-  o.s2 = o.s3 = 0.0;
-  return true;
-}
-
 __global__ void __launch_bounds__(EPC* TPE, 2) k_stiffness_moments(const BlockDev b, const double* __restrict__ X,
                                                                    const double* __restrict__ u,
                                                                    const double* __restrict__ weights, MatDev mat,
@@ -132,6 +82,7 @@ __global__ void __launch_bounds__(EPC* TPE, 2) k_stiffness_moments(const BlockDe
   double acc[45];
 #pragma unroll
   for (int k = 0; k < 45; ++k) acc[k] = 0.0;
+  bool sound = true;  // no doubtful determinant at this thread's points
   for (int q0 = 0; q0 < b.nq; q0 += QT) {
     const int q = q0 + sub;
     if (q0 > 0) __syncthreads();  // the previous tile has been summed
@@ -185,38 +136,38 @@ __global__ void __launch_bounds__(EPC* TPE, 2) k_stiffness_moments(const BlockDe
       const double mu = b.emat ? b.emat[2 * e] : mat.mu, lam = b.emat ? b.emat[2 * e + 1] : mat.lambda;
       QpPair<double> qp;
       double M1[9];
-      if (detJ == 0.0 || !point_state(mat.kind, F, mu, lam, qp, M1)) {
-        s_ok[el] = 0;
-      } else {
-        const double sc = sqrt(b.qw[q] * fabs(detJ));
-        double v[3][9];
+      double scale = 0.0;
 #pragma unroll
-        for (int x = 0; x < 3; ++x) {
+      for (int k = 0; k < 9; ++k) scale = fmax(scale, fabs(J[k]));
+      sound &= point_state(mat.kind, F, mu, lam, qp, M1) && !det_doubtful(detJ, Ji, scale);
+      const double sc = sqrt(b.qw[q] * fabs(detJ));
+      double v[3][9];
 #pragma unroll
-          for (int k = 0; k < 3; ++k) v[x][k] = g[x][k] * sc;
-          mat3vec(F, v[x], v[x] + 3);
-          mat3vec(M1, v[x], v[x] + 6);
-        }
-        double* o = sA + (size_t)sub * AS;
-        // diagonal blocks 11, 22, 33 (upper entries), then 12, 13, 23
+      for (int x = 0; x < 3; ++x) {
 #pragma unroll
-        for (int x = 0; x < 3; ++x) {
-          double k9[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-          pair_block(mat.kind, qp, v[x], v[x], k9);
-          o[6 * x] = k9[0];
-          o[6 * x + 1] = k9[1];
-          o[6 * x + 2] = k9[2];
-          o[6 * x + 3] = k9[4];
-          o[6 * x + 4] = k9[5];
-          o[6 * x + 5] = k9[8];
-        }
+        for (int k = 0; k < 3; ++k) v[x][k] = g[x][k] * sc;
+        mat3vec(F, v[x], v[x] + 3);
+        mat3vec(M1, v[x], v[x] + 6);
+      }
+      double* o = sA + (size_t)sub * AS;
+      // diagonal blocks 11, 22, 33 (upper entries), then 12, 13, 23
 #pragma unroll
-        for (int n = 0; n < 3; ++n) {
-          double k9[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-          pair_block(mat.kind, qp, v[n < 2 ? 0 : 1], v[n == 0 ? 1 : 2], k9);
+      for (int x = 0; x < 3; ++x) {
+        double k9[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+        pair_block(mat.kind, qp, v[x], v[x], k9);
+        o[6 * x] = k9[0];
+        o[6 * x + 1] = k9[1];
+        o[6 * x + 2] = k9[2];
+        o[6 * x + 3] = k9[4];
+        o[6 * x + 4] = k9[5];
+        o[6 * x + 5] = k9[8];
+      }
 #pragma unroll
-          for (int k = 0; k < 9; ++k) o[18 + 9 * n + k] = k9[k];
-        }
+      for (int n = 0; n < 3; ++n) {
+        double k9[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+        pair_block(mat.kind, qp, v[n < 2 ? 0 : 1], v[n == 0 ? 1 : 2], k9);
+#pragma unroll
+        for (int k = 0; k < 9; ++k) o[18 + 9 * n + k] = k9[k];
       }
     }
     __syncthreads();
@@ -270,6 +221,9 @@ __global__ void __launch_bounds__(EPC* TPE, 2) k_stiffness_moments(const BlockDe
 #pragma unroll
           for (int j = 0; j < 3; ++j) o[9 * sym4(x, y) + 3 * i + j] = at(x, y, i, j);
   }
+  if (!sound)
+    for (int q = sub; q < b.nq; q += TPE)
+      if (tet10_singular(mat.kind, s_x[el], s_u[el], b.qp + 3 * (size_t)q)) s_ok[el] = 0;
   __syncthreads();
   // ---- C ---- (a thread decodes the terms of one pair's row once, for half of
   // the CTA's elements)
