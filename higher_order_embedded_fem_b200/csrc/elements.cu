@@ -1,5 +1,7 @@
 // Element kernels: tangent stiffness fused with the colored CSR scatter, and
-// the consistent mass matrix (FP64); the internal forces are in forces.cu.
+// the consistent mass matrix (FP64).  The internal forces are in forces.cu, FP64
+// Hex27 stiffness in stiffness_hex27.cu, staged FP64 Tet10 stiffness of one rule in
+// stiffness_moments.cu, FP32 Tet10 stiffness in stiffness_tc.cu.
 //
 // Reference: fenris/src/assembly.rs:618-797 (element mass / elliptic term /
 // stiffness), :252-314 + :1042-1075 (colored CSR scatter); materials in
@@ -414,7 +416,7 @@ void launch_stiffness_staged(const Model& m, const Block& blk, const MatDev& mat
                              cudaStream_t s) {
   init_pairs();
   if (blk.kind == HOEFEM_ELEM_TET10) launch_stiffness_kind<10, double>(m, blk, mat, u, nullptr, s, stage);
-  else launch_stiffness_kind<27, double>(m, blk, mat, u, nullptr, s, stage);
+  else if (blk.ne > 0) launch_stiffness_hex27(m, blk, nullptr, (int)blk.ne, mat, u, nullptr, stage, nullptr, s);
   HOEFEM_CUDA(cudaGetLastError());
 }
 
@@ -442,7 +444,7 @@ void launch_stiffness(const Model& m, const MatDev& mat, const double* u, double
         else launch_stiffness_kind<10, double>(m, *bp, mat, u, nullptr, s, nullptr, (double*)pb);
       } else {
         if (f32) launch_stiffness_kind<27, float>(m, *bp, mat, u, nullptr, s, nullptr, (float*)pb);
-        else launch_stiffness_kind<27, double>(m, *bp, mat, u, nullptr, s, nullptr, (double*)pb);
+        else launch_stiffness_hex27(m, *bp, nullptr, (int)bp->ne, mat, u, nullptr, nullptr, (double*)pb, s);
       }
       HOEFEM_CUDA(cudaGetLastError());
       stiffness_gather_pairs(m, *bp, f32, vals, store, s);
@@ -453,7 +455,9 @@ void launch_stiffness(const Model& m, const MatDev& mat, const double* u, double
       else launch_stiffness_kind<10, double>(m, *bp, mat, u, vals, s);
     } else {
       if (f32) launch_stiffness_kind<27, float>(m, *bp, mat, u, vals, s);
-      else launch_stiffness_kind<27, double>(m, *bp, mat, u, vals, s);
+      else for_each_color(*bp, [&](const int* elems, int cnt) {
+        launch_stiffness_hex27(m, *bp, elems, cnt, mat, u, vals, nullptr, nullptr, s);
+      });
     }
   }
   HOEFEM_CUDA(cudaGetLastError());

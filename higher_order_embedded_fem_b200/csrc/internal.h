@@ -237,6 +237,11 @@ void stiffness_gather_pairs(const Model& m, const Block& blk, bool f32, double* 
 bool stiffness_moments_eligible(const Block& blk);
 void launch_stiffness_moments(const Model& m, const Block& blk, const MatDev& mat, const double* u, double* pblk,
                               cudaStream_t s);
+// FP64 stiffness of count Hex27 elements (elems, or all by number) on the FP64
+// tensor cores (stiffness_hex27.cu): into node-pair blocks, dense element matrices
+// or, for the elements of a color, added into the CSR values.
+void launch_stiffness_hex27(const Model& m, const Block& blk, const int* elems, int count, const MatDev& mat,
+                            const double* u, double* vals, double* stage, double* pblk, cudaStream_t s);
 // Staged element forces of a whole block (same eligibility): the buffer
 // (element-major node forces) and the per-node gather adding into f.
 double* forces_stage_buffer(const Model& m, const Block& blk, cudaStream_t s);
