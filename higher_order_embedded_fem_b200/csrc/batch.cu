@@ -58,7 +58,9 @@ struct SegCg {
 // writes its chunk's partial sums cpart[k * nch + c].  The per-scene sums add
 // a scene's chunk partials in chunk order: deterministic, and independent of
 // the other scenes.
-constexpr int CHN = 256;
+// (Eight nodes a warp: with 32, the few scenes that run longest left most of the chip
+// idle; a chunk of 32 nodes costs more than it spreads, 85 against 83 ms a step.)
+constexpr int CHN = 64;
 
 struct Chunks {
   const int* lo;     // nch + 1
@@ -241,6 +243,74 @@ __device__ __forceinline__ void node_row_dot_x(const NodeRows& A, const double* 
   }
 }
 
+// The row sums of the nodes lo .. hi of a chunk: body(node, s) in lane 0 of a warp's
+// lanes (lane 0 of the group for narrower variants).  With a warp per node it holds
+// the row descriptions of all its nodes from the start (a lane each) and takes two
+// nodes at a time: their loads overlap, and one of the three dependent loads of a
+// node (offset, neighbour, operand) is off the chain.
+template <int L, class X, class F>
+__device__ __forceinline__ void chunk_rows(const NodeRows& A, const double* __restrict__ vals, const X& x, int lo, int hi,
+                                           F&& body) {
+  if constexpr (L == 32) {
+    static_assert(CHN / (TPB / 32) <= 32, "a lane per node of the warp");
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    constexpr int NW = TPB / 32;
+    const int mine = lo + w + lane * NW;
+    long long base = 0;
+    int off = 0, deg = 0;
+    if (mine < hi) {
+      base = A.base[mine];
+      off = A.adj_off[mine];
+      deg = A.diag_only && A.diag_only[mine] ? -1 : A.adj_off[mine + 1] - off;
+    }
+    for (int k = 0; lo + w + k * NW < hi; k += 2) {
+      const double* r[2];
+      const int* nb[2];
+      int d[2];
+      double s[2][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        r[j] = vals + __shfl_sync(0xffffffffu, base, k + j);
+        nb[j] = A.adj + __shfl_sync(0xffffffffu, off, k + j);
+        d[j] = __shfl_sync(0xffffffffu, deg, k + j);
+        const int a = lo + w + (k + j) * NW;
+        if (d[j] < 0 && lane == 0) {
+#pragma unroll
+          for (int i = 0; i < 3; ++i) s[j][i] = r[j][i] * x(3LL * a + i);
+        }
+      }
+      for (int t = lane; t < max(d[0], d[1]); t += 32) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          if (t >= d[j]) continue;
+          const long long n = nb[j][t];
+          const double x0 = x(3 * n), x1 = x(3 * n + 1), x2 = x(3 * n + 2);
+          const double* r0 = r[j] + 3 * t;
+          const double* r1 = r0 + 3 * d[j];
+          const double* r2 = r1 + 3 * d[j];
+          s[j][0] += r0[0] * x0 + r0[1] * x1 + r0[2] * x2;
+          s[j][1] += r1[0] * x0 + r1[1] * x1 + r1[2] * x2;
+          s[j][2] += r2[0] * x0 + r2[1] * x1 + r2[2] * x2;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int a = lo + w + (k + j) * NW;
+        if (a >= hi) break;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) s[j][i] = warp_sum_d(s[j][i]);
+        if (lane == 0) body(a, s[j]);
+      }
+    }
+  } else {
+    for_chunk_nodes<L>(lo, hi, [&](int a, int sl) {
+      double s[3];
+      node_row_dot_x<L>(A, vals, x, a, sl, s[0], s[1], s[2]);
+      if (a >= 0 && sl == 0) body(a, s);
+    });
+  }
+}
+
 // ---- per-chunk CG steps (chunk c of a running scene, the whole CTA) --------------
 
 // r = b - A x ; chunk partials b.b, r.r
@@ -250,17 +320,13 @@ __device__ __forceinline__ void chunk_init(const NodeRows& A, const double* __re
                                            double* __restrict__ r, const Chunks ch, double* __restrict__ cpart, int c) {
   double acc[2] = {0.0, 0.0};
   const XVec xv{x};
-  for_chunk_nodes<L>(ch.lo[c], ch.lo[c + 1], [&](int a, int sl) {
-    double s[3];
-    node_row_dot_x<L>(A, vals, xv, a, sl, s[0], s[1], s[2]);
-    if (a >= 0 && sl == 0) {
+  chunk_rows<L>(A, vals, xv, ch.lo[c], ch.lo[c + 1], [&](int a, const double (&s)[3]) {
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        double bi = b[3 * a + i], ri = bi - s[i];
-        r[3 * a + i] = ri;
-        acc[0] = fma(bi, bi, acc[0]);
-        acc[1] = fma(ri, ri, acc[1]);
-      }
+    for (int i = 0; i < 3; ++i) {
+      double bi = b[3 * a + i], ri = bi - s[i];
+      r[3 * a + i] = ri;
+      acc[0] = fma(bi, bi, acc[0]);
+      acc[1] = fma(ri, ri, acc[1]);
     }
   });
   chunk_store<2>(acc, cpart, ch.n, c);
@@ -287,17 +353,13 @@ __device__ __forceinline__ void chunk_Ap(const NodeRows& A, const double* __rest
                                          double* __restrict__ pout, double* __restrict__ Ap, const Chunks ch,
                                          double* __restrict__ cpart, int c) {
   double acc[2] = {0.0, 0.0};
-  for_chunk_nodes<L>(ch.lo[c], ch.lo[c + 1], [&](int a, int sl) {
-    double s[3];
-    node_row_dot_x<L>(A, vals, pa, a, sl, s[0], s[1], s[2]);
-    if (a >= 0 && sl == 0) {
+  chunk_rows<L>(A, vals, pa, ch.lo[c], ch.lo[c + 1], [&](int a, const double (&s)[3]) {
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        const double pi = pa(3LL * a + i);
-        if (pout) pout[3 * a + i] = pi;
-        Ap[3 * a + i] = s[i];
-        acc[0] = fma(pi, s[i], acc[0]);
-      }
+    for (int i = 0; i < 3; ++i) {
+      const double pi = pa(3LL * a + i);
+      if (pout) pout[3 * a + i] = pi;
+      Ap[3 * a + i] = s[i];
+      acc[0] = fma(pi, s[i], acc[0]);
     }
   });
   chunk_store<2>(acc, cpart, ch.n, c);
@@ -342,8 +404,12 @@ __global__ void __launch_bounds__(TPB) k_seg_prec0(const Chunks ch, const SegCg*
   chunk_prec0(ch, d, r, z, p, cpart, c);
 }
 
+// Bound by the matrix while many scenes run (64 scenes, 149 M values: 315 -> 258 us,
+// 4.6 TB/s), by the latency of a chunk's node loop when few do (125 -> 42 us).  Five
+// CTAs per SM: four leave too few loads in flight (313 us), six take the registers
+// of the second node (277).
 template <int L>
-__global__ void __launch_bounds__(TPB) k_seg_Ap(NodeRows A, const double* __restrict__ vals,
+__global__ void __launch_bounds__(TPB, 5) k_seg_Ap(NodeRows A, const double* __restrict__ vals,
                                                 const double* __restrict__ p, double* __restrict__ Ap, const Chunks ch,
                                                 const SegCg* __restrict__ st, double* __restrict__ cpart) {
   const int c = blockIdx.x;
