@@ -126,6 +126,7 @@ __device__ void hex_half_space(const Hex& h, int f, P3& x0, P3& n) {
 // ---- the clipped polyhedron of one (cell, tet) pair ---------------------------
 struct Poly {
   int nv, nf;
+  bool labelled;  // vertices are labelled by first appearance over the faces
   P3 X[EMV];
   unsigned char fn[EMF];
   unsigned char fv[EMF][EMFV];
@@ -148,7 +149,19 @@ __device__ P3 seg_plane(P3 a, P3 b, P3 x0, P3 n) {
 // Keeps the part with n.(x - x0) >= 0.  Returns false on a capacity overflow.
 __device__ bool clip(Poly& P, P3 x0, P3 n) {
   bool in[EMV];
-  for (int v = 0; v < P.nv; ++v) in[v] = dot(n, sub(P.X[v], x0)) >= 0.0;
+  int nin = 0;
+  for (int v = 0; v < P.nv; ++v) {
+    in[v] = dot(n, sub(P.X[v], x0)) >= 0.0;
+    nin += in[v];
+  }
+  // nothing left, or nothing cut off and nothing to relabel: most pairs' boxes meet
+  // where the cells do not, and most half-spaces do not cut the rest (counting pass of
+  // 13,824 cells and 186,624 tets 10.5 -> 6.4 ms)
+  if (nin == 0) {
+    P.nv = P.nf = 0;
+    return true;
+  }
+  if (nin == P.nv && P.labelled) return true;
   unsigned short R[EMF][EMFV];
   unsigned char rn[EMF];
   int nr = 0;
@@ -239,6 +252,7 @@ __device__ bool clip(Poly& P, P3 x0, P3 n) {
     newn[nf] = rn[f];
     ++nf;
   }
+  P.labelled = true;
   P.nv = nl;
   for (int v = 0; v < nl; ++v) P.X[v] = Y[v];
   P.nf = nf;
@@ -267,6 +281,7 @@ __device__ bool clip_pair(const Hex& h, const double* __restrict__ eX, const int
       g[j] = g[j - 1];
       g[j - 1] = tmp;
     }
+  P.labelled = false;
   P.nv = ng;
   for (int i = 0; i < ng; ++i) P.X[i] = mk(eX[3 * (size_t)g[i]], eX[3 * (size_t)g[i] + 1], eX[3 * (size_t)g[i] + 2]);
   P.nf = 4;
@@ -394,42 +409,76 @@ __device__ bool hex_inverse(const Hex& h, P3 x, P3& xi) {
 }
 
 // ---- kernels -------------------------------------------------------------------
+constexpr int CTILE = 256;  // consecutive tets of a tile
+
+// Bounding box of every tile of tets (one warp per tile).
+__global__ void __launch_bounds__(128) k_embed_tiles(long long nt, const double* __restrict__ tbox,
+                                                     double* __restrict__ tile) {
+  const int lane = threadIdx.x & 31;
+  const long long g = blockIdx.x * 4LL + (threadIdx.x >> 5);
+  const long long lo = g * CTILE, hi = min(lo + CTILE, nt);
+  if (lo >= hi) return;
+  double b[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  for (long long t = lo + lane; t < hi; t += 32)
+    for (int k = 0; k < 3; ++k) {
+      b[k] = fmin(b[k], tbox[6 * t + k]);
+      b[3 + k] = fmax(b[3 + k], tbox[6 * t + 3 + k]);
+    }
+  for (int k = 0; k < 3; ++k)
+    for (int o = 16; o > 0; o >>= 1) {
+      b[k] = fmin(b[k], __shfl_xor_sync(0xffffffffu, b[k], o));
+      b[3 + k] = fmax(b[3 + k], __shfl_xor_sync(0xffffffffu, b[3 + k], o));
+    }
+  if (lane < 6) tile[6 * g + lane] = lane == 0 ? b[0] : lane == 1 ? b[1] : lane == 2 ? b[2] : lane == 3 ? b[3] : lane == 4 ? b[4] : b[5];
+}
+
+__device__ __forceinline__ bool boxes_meet(const double* a, const double* b) {
+  return a[0] <= b[3] && b[0] <= a[3] && a[1] <= b[4] && b[1] <= a[4] && a[2] <= b[5] && b[2] <= a[5];
+}
+
 // Candidate tets of every cell (bounding boxes meet, closed intervals), in
-// ascending tet order: count pass (out == nullptr) or fill pass.
-__global__ void __launch_bounds__(256) k_embed_candidates(long long nbc, const double* __restrict__ cbox,
-                                                          long long nt, const double* __restrict__ tbox,
-                                                          const long long* __restrict__ off, long long* __restrict__ count,
-                                                          int* __restrict__ out) {
-  __shared__ int s_w[8];
-  __shared__ long long s_base;
+// ascending tet order: count pass (out == nullptr) or fill pass.  One CTA per cell;
+// only the tiles whose box meets the cell's are looked through (13,824 cells, 186,624
+// tets: 6.9 ms a pass with every tet's box read for every cell, 0.12 now; eight cells
+// to a CTA that reads them all, 5.3).
+__global__ void __launch_bounds__(CTILE) k_embed_candidates(long long nbc, const double* __restrict__ cbox,
+                                                            long long nt, const double* __restrict__ tbox,
+                                                            const double* __restrict__ tile,
+                                                            const long long* __restrict__ off, long long* __restrict__ count,
+                                                            int* __restrict__ out) {
+  __shared__ unsigned s_hit[CTILE / 32];
+  __shared__ int s_w[2][CTILE / 32];
   const long long c = blockIdx.x;
   if (c >= nbc) return;
   double cb[6];
   for (int k = 0; k < 6; ++k) cb[k] = cbox[6 * c + k];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (threadIdx.x == 0) s_base = out ? off[c] : 0;
-  __syncthreads();
-  for (long long t0 = 0; t0 < nt; t0 += blockDim.x) {
-    const long long t = t0 + threadIdx.x;
-    bool hit = false;
-    if (t < nt) {
-      const double* tb = tbox + 6 * t;
-      hit = cb[0] <= tb[3] && tb[0] <= cb[3] && cb[1] <= tb[4] && tb[1] <= cb[4] && cb[2] <= tb[5] && tb[2] <= cb[5];
-    }
-    const unsigned bal = __ballot_sync(0xffffffffu, hit);
-    if (lane == 0) s_w[w] = __popc(bal);
+  long long base = out ? off[c] : 0;
+  const long long ntile = (nt + CTILE - 1) / CTILE;
+  int turn = 0;
+  for (long long g0 = 0; g0 < ntile; g0 += CTILE) {
+    const long long g = g0 + threadIdx.x;
+    const unsigned near = __ballot_sync(0xffffffffu, g < ntile && boxes_meet(cb, tile + 6 * g));
+    __syncthreads();  // the previous tiles' bits have been read
+    if (lane == 0) s_hit[w] = near;
     __syncthreads();
-    int before = 0, total = 0;
-    for (int k = 0; k < 8; ++k) {
-      if (k < w) before += s_w[k];
-      total += s_w[k];
-    }
-    if (hit && out) out[s_base + before + __popc(bal & ((1u << lane) - 1u))] = (int)t;
-    __syncthreads();
-    if (threadIdx.x == 0) s_base += total;
-    __syncthreads();
+    for (int k = 0; k < CTILE / 32; ++k)
+      for (unsigned m = s_hit[k]; m; m &= m - 1, turn ^= 1) {
+        const long long t = (g0 + 32 * k + __ffs((int)m) - 1) * CTILE + threadIdx.x;
+        const bool hit = t < nt && boxes_meet(cb, tbox + 6 * t);
+        const unsigned bal = __ballot_sync(0xffffffffu, hit);
+        if (lane == 0) s_w[turn][w] = __popc(bal);
+        __syncthreads();  // (the other half of s_w may still be read)
+        int before = 0, total = 0;
+        for (int j = 0; j < CTILE / 32; ++j) {
+          if (j < w) before += s_w[turn][j];
+          total += s_w[turn][j];
+        }
+        if (hit && out) out[base + before + __popc(bal & ((1u << lane) - 1u))] = (int)t;
+        base += total;
+      }
   }
-  if (!out && threadIdx.x == 0) count[c] = s_base;
+  if (!out && threadIdx.x == 0) count[c] = base;
 }
 
 // Pass 1: cut volume and tetrahedron count of every pair.
@@ -1148,8 +1197,15 @@ Embedding* embedding_create(const double* bgX, i64 nbv, const i64* bg_conn, i64 
   // candidate pairs
   DBuf<long long> d_count, d_off;
   d_count.alloc(nbc);
-  (note_launch(), k_embed_candidates<<<(unsigned)nbc, 256, 0, s>>>(nbc, d_cbox.p, nt, d_tbox.p, nullptr, d_count.p,
-                                                                   nullptr));
+  DBuf<double> d_tile;
+  const i64 ntile = (nt + CTILE - 1) / CTILE;
+  d_tile.alloc(6 * std::max<i64>(ntile, 1));
+  if (ntile) (note_launch(), k_embed_tiles<<<(unsigned)((ntile + 3) / 4), 128, 0, s>>>(nt, d_tbox.p, d_tile.p));
+  auto candidates = [&](const long long* offsets, long long* counts, int* out) {
+    (note_launch(), k_embed_candidates<<<(unsigned)nbc, CTILE, 0, s>>>(nbc, d_cbox.p, nt, d_tbox.p, d_tile.p, offsets,
+                                                                       counts, out));
+  };
+  candidates(nullptr, d_count.p, nullptr);
   HOEFEM_CUDA(cudaGetLastError());
   std::vector<long long> cnt(nbc);
   HOEFEM_CUDA(cudaMemcpyAsync(cnt.data(), d_count.p, sizeof(long long) * nbc, cudaMemcpyDeviceToHost, s));
@@ -1161,8 +1217,7 @@ Embedding* embedding_create(const double* bgX, i64 nbv, const i64* bg_conn, i64 
   std::vector<long long> offl(E->off.begin(), E->off.end());
   d_off.upload(offl, s);
   E->d_ptet.alloc(E->npairs);
-  (note_launch(), k_embed_candidates<<<(unsigned)nbc, 256, 0, s>>>(nbc, d_cbox.p, nt, d_tbox.p, d_off.p, nullptr,
-                                                                   E->d_ptet.p));
+  candidates(d_off.p, nullptr, E->d_ptet.p);
   std::vector<int> pcell(E->npairs);
   for (i64 c = 0; c < nbc; ++c)
     for (i64 k = E->off[c]; k < E->off[c + 1]; ++k) pcell[k] = (int)c;
