@@ -351,7 +351,6 @@ int hoefem_assemble_elastic_pseudo_forces_into(hoefem_model m, const hoefem_mate
   View U(u, mm.ndof, mem, mm.stream, true), F(f, mm.ndof, mem, mm.stream, true);
   launch_forces(mm, md, U.d, F.d, mm.stream);
   F.copy_out();
-  sync(mm);
   check_device_error(mm);
   API_END
 }
@@ -364,7 +363,6 @@ int hoefem_assemble_stiffness_into(hoefem_model m, const hoefem_material* mat, c
   View U(u, mm.ndof, mem, mm.stream, true), V(values, mm.nnz, mem, mm.stream, true);
   launch_stiffness(mm, md, U.d, V.d, mm.stream);
   V.copy_out();
-  sync(mm);
   check_device_error(mm);
   API_END
 }
@@ -379,7 +377,6 @@ int hoefem_assemble_stiffness_into_precision(hoefem_model m, const hoefem_materi
   View U(u, mm.ndof, mem, mm.stream, true), V(values, mm.nnz, mem, mm.stream, true);
   launch_stiffness(mm, md, U.d, V.d, mm.stream, precision == HOEFEM_PRECISION_MIXED ? PRECISION_FP32 : PRECISION_FP64);
   V.copy_out();
-  sync(mm);
   check_device_error(mm);
   API_END
 }
@@ -392,7 +389,6 @@ int hoefem_assemble_projected_stiffness_into(hoefem_model m, const hoefem_materi
   View U(u, mm.ndof, mem, mm.stream, true), V(values, mm.nnz, mem, mm.stream, true);
   launch_stiffness_projected(mm, md, U.d, V.d, mm.stream);
   V.copy_out();
-  sync(mm);
   check_device_error(mm);
   API_END
 }
@@ -403,7 +399,6 @@ int hoefem_assemble_mass_into(hoefem_model m, double density, double* values, in
   View V(values, mm.nnz, mem, mm.stream, true);
   launch_mass(mm, density, V.d, mm.stream);
   V.copy_out();
-  sync(mm);
   check_device_error(mm);
   API_END
 }

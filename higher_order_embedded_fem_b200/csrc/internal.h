@@ -185,6 +185,7 @@ struct Model {
   DBuf<unsigned> d_sched;  // SpMV dynamic-scheduling counters (zero between launches)
   DBuf<double> d_stage;    // dense element matrices (projected stiffness), allocated on first use
   DBuf<long long> d_base;
+  int* h_err = nullptr;    // page-locked copy of d_err
   int spmv_lanes = 32;    // SpMV variant for FP64 values (autotuned)
   int spmv_lanes32 = 0;   // SpMV variant for FP32 values (0: as spmv_lanes)
   bool spmv_pinned = false;  // set explicitly by the caller: no autotuning
@@ -278,6 +279,7 @@ void export_pattern(const std::vector<int>& adj_off, const std::vector<int>& adj
                     const std::vector<unsigned char>* diag_only, i64 nv, int64_t* ro, int64_t* ci);
 
 // ---- errors ----------------------------------------------------------------
-void check_device_error(const Model& m);  // reads and clears d_err
+// Waits for the model's stream, reads d_err and clears it; throws if it was set.
+void check_device_error(const Model& m);
 
 }  // namespace hoefem
