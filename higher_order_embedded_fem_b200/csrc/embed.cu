@@ -803,16 +803,17 @@ __device__ __forceinline__ void simp_setup(SimpCta& C, int n, const double* __re
 // the (value, place) reductions are three integer ones over the bits of non-negative
 // doubles.  The element-by-element form spends some 11,000 warp instructions per
 // dropped point on 20 moments (indices, operands and results of every update through
-// shared memory), this one some 3,900 at 24 warps per SM, bound by their latency:
-// 7.7 M points of 3,072 rules, 116 -> 58 ms.
+// shared memory), this one some 3,900 at 32 warps per SM, bound by their latency:
+// 7.7 M points of 3,072 rules, 116 -> 56 ms (68 at 16 warps, 58 at 24).
 template <int R>
 struct SimpWarp {
-  double U[R][R + 2 + (R & 1)];  // pivot rows
+  double U[R * (R + 3) / 2];     // pivot rows k: columns k .. R (row(k)[j])
   double T[2 * R][10];           // per list entry: 1, T_1..3(x), T_1..3(y), T_1..3(z)
   double w[2 * R];
   int idx[2 * R];   // point of the entry
   int list[2 * R];  // entries in order
   int pv[R];
+  __device__ __forceinline__ double* row(int k) { return U + k * (R + 1) - k * (k + 1) / 2; }
 };
 
 // Smallest place among the lanes with the largest v >= 0 (`in` lanes only; limit if none).
@@ -867,18 +868,19 @@ __device__ __forceinline__ int warp_reduce_rows(const SimpCta& C, SimpWarp<R>& S
         const double best = redux_argmax(v, place >= row && place < R && v >= 0.0, place, R, at);
         if (best > eps) {
           const bool pivot = place == at;
+          double* u = S.row(row);
           if (place == row) place = at;
           if (pivot) {
             place = row;
 #pragma unroll
-            for (int j = c; j < M; ++j) S.U[row][j] = A[j];
+            for (int j = c; j < M; ++j) u[j] = A[j];
             S.pv[row] = c;
           }
           __syncwarp();
           if (place > row && place < R) {
-            const double z = A[c] / S.U[row][c];
+            const double z = A[c] / u[c];
 #pragma unroll
-            for (int j = c + 1; j < M; ++j) A[j] = __dsub_rn(A[j], __dmul_rn(z, S.U[row][j]));
+            for (int j = c + 1; j < M; ++j) A[j] = __dsub_rn(A[j], __dmul_rn(z, u[j]));
           }
           pivmask |= 1u << c;
           ++row;
@@ -893,14 +895,15 @@ __device__ __forceinline__ int warp_reduce_rows(const SimpCta& C, SimpWarp<R>& S
     }
     double z = lane == 31 - __clz((int)freemask) ? 1.0 : 0.0;
     for (int k = row - 1; k >= 0; --k) {
+      const double* u = S.row(k);
       const int c = S.pv[k], n = M - 1 - c;  // n terms, in lanes 0 .. n - 1
       const double zj = __shfl_sync(0xffffffffu, z, (c + 1 + lane) & 31);
-      double s = lane < n ? __dmul_rn(S.U[k][c + 1 + lane], zj) : 0.0;
+      double s = lane < n ? __dmul_rn(u[c + 1 + lane], zj) : 0.0;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1)
         if (n > o) s += __shfl_xor_sync(0xffffffffu, s, o);
       s = __shfl_sync(0xffffffffu, s, 0);
-      const double zc = -s / S.U[k][c];
+      const double zc = -s / u[c];
       if (lane == c) z = zc;
     }
     // direction: flipped when no component is positive
@@ -945,7 +948,7 @@ __device__ __forceinline__ int warp_reduce_rows(const SimpCta& C, SimpWarp<R>& S
 constexpr int SIMP_ROWS_WARPS = 8;
 
 template <int R>
-__global__ void __launch_bounds__(32 * SIMP_ROWS_WARPS, 3) k_simplify_rows(const long long* __restrict__ off, const double* __restrict__ p,
+__global__ void __launch_bounds__(32 * SIMP_ROWS_WARPS, 4) k_simplify_rows(const long long* __restrict__ off, const double* __restrict__ p,
                                                        double* __restrict__ wk, int strength, int* __restrict__ grp,
                                                        int* __restrict__ gcnt, int* __restrict__ keep,
                                                        int* __restrict__ nkeep, int* err) {
