@@ -15,7 +15,7 @@
 // 15 weighted sums of them over the points.  Per element of the 14-point rule
 // 14 x (560 + 45 x 15) + 3,000 operations instead of 55 x 14 x 62, and the pair
 // loop's operands are no longer read from shared memory per pair (31
-// loads for 60 FMAs, which bound it).  201,600 elements: 2.56 -> 0.86 ms (0.8 GB
+// loads for 60 FMAs, which bound it).  201,600 elements: 2.56 -> 0.81 ms (0.8 GB
 // of blocks written; eight warps per SM fit, so it is bound by their latency).
 // Relative error against 64-bit torch 3e-16, as the pair loop's (2e-16).
 //
@@ -49,7 +49,10 @@ constexpr int BSE = NW * 90 + 2;
 constexpr int NPAIR = 55;
 
 // place of a symmetric 4 x 4 index pair x <= y: 00 01 02 03 11 12 13 22 23 33
-__host__ __device__ constexpr int sym4(int x, int y) { return x <= y ? 4 * x - x * (x - 1) / 2 + y - x : sym4(y, x); }
+__host__ __device__ constexpr int sym4(int x, int y) {
+  const int lo = x < y ? x : y, hi = x < y ? y : x;
+  return 4 * lo - lo * (lo - 1) / 2 + hi - lo;
+}
 
 // Four terms per node pair: offset of the block in the element's array (m * 90
 // + 9 * block), bit 11 set if it is read transposed, and the coefficient + 8
