@@ -410,7 +410,7 @@ def run_hoefem(args):
 
 
 def cg_roofline(var, head, fp16=False):
-    """Streamed CG of one variant: algorithmic bytes per iteration = operator
+    """CG of one variant (streamed: as follows): algorithmic bytes per iteration = operator
     tiles (values + neighbour lists + tile headers) + Schwarz block chunks, the
     data an iteration must read from HBM (vectors, 1 MB each, stay in L2);
     achieved = bytes x iterations / summed device time of the persistent
@@ -418,9 +418,18 @@ def cg_roofline(var, head, fp16=False):
     eng = var.get("cg_engine") or {}
     peaks_path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     peak = json.load(open(peaks_path))["hbm_gbs"] if os.path.exists(peaks_path) else 6650.0
+    per_it = eng.get("operator_bytes", 0) + eng.get("schwarz_bytes", 0)
+    if eng.get("auto_choice") == 0 and not eng.get("launches") and per_it and var.get("cg_iterations"):
+        # the solves ran as persistent launches on the CSR values: the same
+        # bytes (up to list widths) over the whole CG phase of the step
+        ms_it = var["phase_ms"]["cg"] / var["cg_iterations"]
+        gbs = per_it / (ms_it * 1e-3) / 1e9
+        return {"kernel": "k_pcg (persistent Schwarz-PCG on the CSR values)", "bound": "hbm", "achieved": gbs,
+                "peak": peak, "unit": "GB/s", "frac": gbs / peak, "traffic": None, "bytes_per_iteration": per_it,
+                "us_per_iteration": ms_it * 1e3, "iterations": var["cg_iterations"],
+                "peak_source": "measured" if os.path.exists(peaks_path) else "fallback"}
     if not eng.get("launches") or not eng.get("iterations") or not eng.get("device_ms"):
         return None
-    per_it = eng["operator_bytes"] + eng["schwarz_bytes"]
     ms_it = eng["device_ms"] / eng["iterations"]
     gbs = per_it / (ms_it * 1e-3) / 1e9
     kern = {"plain": "k_cg_stream<double,double,2>", "mixed": "k_cg_stream<float,float,2>",
