@@ -27,6 +27,7 @@
 #include <cmath>
 #include <cstdint>
 
+#include "cg_limit.h"
 #include "internal.h"
 #include "kernels_common.cuh"
 #include "learned.h"
@@ -691,7 +692,10 @@ int run_pcg(CgWork& w, Operator A, const Precond* P, bool p32, double tol, i64 m
   if (w.stream_mode == 0 && et.choice < 0) HOEFEM_CUDA(cudaEventRecord(w.tev[0], s));
   CgState init{};
   init.tol = tol;
-  init.max_iter = max_iter;
+  // on the device every solve has a limit: the persistent kernels run until they
+  // have reached it
+  init.max_iter = cg_iteration_limit(max_iter, n, w.chunk);
+  const i64 max_chunks = cg_max_chunks(max_iter, n, w.chunk);
   HOEFEM_CUDA(cudaMemcpyAsync(w.st.p, &init, sizeof(CgState), cudaMemcpyHostToDevice, s));
   const int vg = vec_grid(n);
   HOEFEM_REQUIRE(R.sched, HOEFEM_ERR_INVALID_ARGUMENT, "node-row matrix without scheduling counters");
@@ -776,8 +780,7 @@ int run_pcg(CgWork& w, Operator A, const Precond* P, bool p32, double tol, i64 m
     // one launch per residual replacement
     cg_stream_arm(w, A64 ? delta : 0.0, s);
     w.stream_ms = 0.f;
-    const i64 cap_s = max_iter >= 0 ? max_iter : 10 * (i64)n;
-    i64 nrep_s = 0;
+    i64 nrep_s = 0, chunks = 0;
     for (;;) {
       const i64 it0 = w.h_st->iters;
       if (streamed) {
@@ -789,6 +792,7 @@ int run_pcg(CgWork& w, Operator A, const Precond* P, bool p32, double tol, i64 m
       // a launch that ran no iteration found the solve finished by the
       // replacement before it
       const bool ran = w.h_st->iters > it0;
+      chunks += cg_chunks_of(w.h_st->iters - it0, w.chunk);
       if (A64 && ran) {
         const bool conv = w.h_st->done && w.h_st->status == HOEFEM_OK;
         const bool trig = !w.h_st->done && w.h_st->replace;
@@ -811,11 +815,13 @@ int run_pcg(CgWork& w, Operator A, const Precond* P, bool p32, double tol, i64 m
             HOEFEM_CUDA(cudaStreamSynchronize(s));
             if (w.h_st->done) break;
           }
-          continue;
+          // without a limit of the caller's, replacements that the true residual
+          // keeps asking for end as in the graphs' loop
+          if (max_iter >= 0 || chunks < max_chunks) continue;
         }
       }
       if (w.h_st->done) break;
-      if (w.h_st->iters >= cap_s) {
+      if (chunks >= max_chunks) {
         if (replacements) *replacements = nrep_s;
         *iters = w.h_st->iters;
         return HOEFEM_CG_MAX_ITERATIONS;
@@ -847,9 +853,6 @@ int run_pcg(CgWork& w, Operator A, const Precond* P, bool p32, double tol, i64 m
       else Pm->spmv_lanes = lp;
     }
   };
-  // without an iteration limit CG is still bounded: 10 n iterations
-  const i64 cap = max_iter >= 0 ? max_iter : 10 * (i64)n;
-  const i64 max_chunks = (cap + w.chunk - 1) / w.chunk + 2;
   double rr_ref = w.h_st->rr;
   // the engine sample of this solve counts only if the SpMV variants were already tuned
   const bool sample_chunked = tu.done;

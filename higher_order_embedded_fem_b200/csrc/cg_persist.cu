@@ -58,6 +58,7 @@
 
 #include <algorithm>
 
+#include "cg_limit.h"
 #include "internal.h"
 #include "pcg_layout.h"
 #include "solver.h"
@@ -382,7 +383,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_pcg(const Args A) {
   double zTr = st0->zTr, beta = st0->beta, alpha = st0->alpha, pAp = st0->pAp, rr = st0->rr;
   const double bnorm = st0->bnorm, tol = st0->tol, rr_ref = st0->rr_ref, delta2 = st0->delta2;
   long long iters = st0->iters;
-  const long long max_iter = st0->max_iter;
+  const long long limit = st0->max_iter;  // never negative (cg_limit.h)
   int status = HOEFEM_OK, done = 0, replace = 0;
   const int na = (int)((long long)A.nv * c / G), nb = (int)((long long)A.nv * (c + 1) / G);
   X* px = reinterpret_cast<X*>(A.px);
@@ -608,12 +609,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_pcg(const Args A) {
         stepped = true;
       }
     }
-    iters += 1;
-    if (sqrt(rr) <= tol * bnorm) {
+    if (cg_iteration_end(alpha, rr, tol, bnorm, limit, iters, status)) {
       done = 1;
-    } else if (max_iter >= 0 && iters >= max_iter) {
-      done = 1;
-      status = HOEFEM_CG_MAX_ITERATIONS;
     } else {
       beta = zr / zTr;
       zTr = zr;

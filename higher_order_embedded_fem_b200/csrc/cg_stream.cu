@@ -55,6 +55,7 @@
 #include <cmath>
 #include <vector>
 
+#include "cg_limit.h"
 #include "internal.h"
 #include "kernels_common.cuh"
 #include "solver.h"
@@ -335,7 +336,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_cg_stream(Args A) {
   double zTr = st->zTr, beta = st->beta, alpha = st->alpha, pAp = st->pAp, rr = st->rr;
   const double bnorm = st->bnorm, tol = st->tol, rr_ref = st->rr_ref, delta2 = st->delta2;
   long long iters = st->iters;
-  const long long max_iter = st->max_iter;
+  const long long limit = st->max_iter;  // never negative (cg_limit.h)
   int status = HOEFEM_OK, done = 0, replace = 0, pcur = 0, rcur = 0;
   long long it = 0;
   const int grp = lane >> 3, gl = lane & 7;  // operator tiles: node group and its lane
@@ -593,18 +594,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_cg_stream(Args A) {
     tock(9, tu);
     rr = s_bc[1];
     const double zr = s_bc[2];
-    iters += 1;
     ++it;
     pcur = (int)(it & 1);
     rcur = (int)(it & 1);
-    if (sqrt(rr) <= tol * bnorm) {
+    if (cg_iteration_end(alpha, rr, tol, bnorm, limit, iters, status)) {
       done = 1;
-      status = HOEFEM_OK;
-      break;
-    }
-    if (max_iter >= 0 && iters >= max_iter) {
-      done = 1;
-      status = HOEFEM_CG_MAX_ITERATIONS;
       break;
     }
     beta = zr / zTr;

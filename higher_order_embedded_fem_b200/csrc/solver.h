@@ -78,7 +78,7 @@ void precond_to_fp32(Precond& p, cudaStream_t s);
 
 struct CgState {
   double bnorm, tol, zTr, pAp, rr, alpha, beta;
-  long long iters, max_iter;
+  long long iters, max_iter;  // (of run_pcg: never negative, cg_limit.h)
   int done, status;
   // streamed CG: residual-replacement trigger (rr <= delta2 * rr_ref), the
   // flag it raises, and which direction buffer holds the current direction

@@ -270,7 +270,10 @@ int hoefem_precond_destroy(hoefem_precond p);
    RelativeResidualCriterion (cg.rs:77-124): stops when ||r|| <= tol ||b||.
    x holds the initial guess on entry.  p == NULL means no preconditioner.
    Returns HOEFEM_OK or one of the HOEFEM_CG_* outcomes; *iterations is always
-   written (CgOutput::num_iterations). */
+   written (CgOutput::num_iterations).  max_iter < 0: no limit of the caller's,
+   but a solve that does not converge (a NaN among its numbers, a tolerance below
+   rounding) still ends, as HOEFEM_CG_MAX_ITERATIONS after 10 iterations per
+   unknown, rounded up to chunks of eight, and two chunks. */
 int hoefem_cg_solve(hoefem_model m, const double* system_values, hoefem_precond p, const double* b, double* x,
                     double tol, int64_t max_iter, int64_t* iterations, int mem);
 
