@@ -699,7 +699,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_pcg(const Args A) {
 template <class VA, class VB, int PK>
 void launch(const Args& args, int G, size_t smem, cudaStream_t s) {
   auto fn = k_pcg<VA, VB, PK>;
-  HOEFEM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_shared(fn, SMEM_BUDGET);
   Args a = args;
   void* kargs[] = {&a};
   note_launch();

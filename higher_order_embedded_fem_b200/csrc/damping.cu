@@ -93,7 +93,8 @@ void launch_stiffness_projected(Model& m, const MatDev& mat, const double* u, do
     const int mm = (dim + 1) & ~1;
     const size_t smem = sizeof(double) * (2 * (size_t)mm * mm + mm);
     launch_stiffness_staged(m, *bp, mat, u, m.d_stage.p, s);
-    HOEFEM_CUDA(cudaFuncSetAttribute(k_psd_project, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr size_t MM = 82;  // Hex27: 81 rows, rounded up to even
+    allow_shared(k_psd_project, sizeof(double) * (2 * MM * MM + MM));
     (note_launch(), k_psd_project<<<(int)bp->ne, PSD_TPB, smem, s>>>(dim, m.d_stage.p));
     BlockDev bd = bp->dev();
     const int nc = (int)bp->color_off.size() - 1;

@@ -1387,9 +1387,10 @@ void quadrature_simplify(i64 nrules, const i64* off, const double* w, const doub
       // warps per CTA from the per-warp shared memory (A, z, list, pivots)
       const int m = r + 1, G = 2 * r;
       const size_t per = (size_t)r * m + m + (size_t)(G + m + 1) / 2 + 1;
-      const int nw = (int)std::max<size_t>(1, std::min<size_t>(8, (200 * 1024) / (per * sizeof(double))));
+      constexpr size_t MOST = 200 * 1024;
+      const int nw = (int)std::max<size_t>(1, std::min<size_t>(8, MOST / (per * sizeof(double))));
       const size_t smem = (size_t)nw * per * sizeof(double);
-      HOEFEM_CUDA(cudaFuncSetAttribute(k_simplify, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      allow_shared(k_simplify, MOST);
       (note_launch(), k_simplify<<<(unsigned)nrules, 32 * nw, smem, s>>>(d_off.p, d_p.p, d_w.p, strength, r, d_grp.p,
                                                                           d_gcnt.p, d_keep.p, d_nkeep.p, d_err.p));
     }

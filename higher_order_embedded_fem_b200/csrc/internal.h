@@ -44,6 +44,15 @@ struct Error : std::runtime_error {
     if (!(cond)) throw ::hoefem::Error((code), (msg)); \
   } while (0)
 
+// The dynamic shared memory a kernel may be launched with.  The limit belongs to the
+// kernel on the device, not to a launch, and models of other host threads launch
+// the same kernel: so `most` is what the kernel can ask for at any size, never one
+// model's share, which would refuse the launch of a larger one.
+template <class K>
+void allow_shared(K* kernel, size_t most) {
+  HOEFEM_CUDA(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+}
+
 // Device buffer owned by a handle (plain cudaMalloc, freed on destruction).
 template <class T>
 struct DBuf {

@@ -546,9 +546,6 @@ void precond_create_schwarz(Precond& p, const i64* sub_off, const i64* sub_nodes
   p.d_sched.zero(st);
   p.d_err.zero(st);
   HOEFEM_CUDA(cudaStreamSynchronize(st));
-  int m_max = (3 * p.max_nodes + 1) & ~1;
-  size_t smem = (size_t)(2 * m_max * m_max + m_max) * sizeof(double);
-  HOEFEM_CUDA(cudaFuncSetAttribute(k_schwarz_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   p.spmv_lanes = autotune_spmv_lanes(p.rows(), p.vals.p, st);
 }
 
@@ -597,7 +594,7 @@ void precond_update(Precond& p, const double* J, cudaStream_t s) {
     const size_t gj_smem = sizeof(double) * (size_t)dmax * (dmax | 1);
 #define HOEFEM_GJ(NT)                                                                                                  \
   do {                                                                                                                 \
-    HOEFEM_CUDA(cudaFuncSetAttribute(k_schwarz_gj<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gj_smem));    \
+    allow_shared(k_schwarz_gj<NT>, sizeof(double) * 9 * NT * (9 * NT | 1));                                            \
     (note_launch(), k_schwarz_gj<NT><<<(int)p.nsub, (NT * NT + 31) / 32 * 32, gj_smem, s>>>(                           \
                         p.d_sub_off.p, p.d_sub_nodes.p, p.d_gmap_off.p, p.d_gmap.p, m.d_adj_off.p, m.d_base.p, J,      \
                         p.d_stage_off.p, p.bsym.p, p.d_fallback.p));                                                   \
@@ -607,8 +604,9 @@ void precond_update(Precond& p, const double* J, cudaStream_t s) {
     else if (p.max_nodes <= 18) HOEFEM_GJ(6);
     else HOEFEM_GJ(9);
 #undef HOEFEM_GJ
-    int m_max = (dmax + 1) & ~1;
-    size_t smem = (size_t)(2 * m_max * m_max + m_max) * sizeof(double);
+    auto factor_smem = [](size_t m2) { return (2 * m2 * m2 + m2) * sizeof(double); };
+    const size_t smem = factor_smem((dmax + 1) & ~1);
+    allow_shared(k_schwarz_factor, factor_smem(82));  // 27 nodes, rounded up to even
     (note_launch(), k_schwarz_factor<<<(int)p.nsub, FACTOR_TPB, smem, s>>>(p.d_fallback.p, p.d_sub_off.p,
                                                                            p.d_sub_nodes.p, p.d_gmap_off.p, p.d_gmap.p,
                                                                            m.d_adj_off.p, m.d_base.p, J, p.d_stage_off.p,
