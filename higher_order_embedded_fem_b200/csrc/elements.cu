@@ -24,6 +24,7 @@
 
 #include "element_math.cuh"
 #include "internal.h"
+#include "pair_tables.h"
 
 namespace hoefem {
 
@@ -43,17 +44,13 @@ constexpr int TPB = 128;
 // Two barriers per tile (one tile for all standard rules), against two per
 // point with a single node-building warp.
 // ============================================================================
-template <int NN>
-struct PairTable {
-  static constexpr int NP = NN * (NN + 1) / 2;
-};
-__constant__ unsigned char c_pairs10[55][2];
-__constant__ unsigned char c_pairs27[378][2];
+__constant__ PairTable<10> c_pairs10 = pair_table<10>();
+__constant__ PairTable<27> c_pairs27 = pair_table<27>();
 
 template <int NN>
 __device__ __forceinline__ void pair_of(int p, int& I, int& J) {
-  if (NN == 10) { I = c_pairs10[p][0]; J = c_pairs10[p][1]; }
-  else { I = c_pairs27[p][0]; J = c_pairs27[p][1]; }
+  if (NN == 10) { I = c_pairs10.at[p][0]; J = c_pairs10.at[p][1]; }
+  else { I = c_pairs27.at[p][0]; J = c_pairs27.at[p][1]; }
 }
 
 template <int NN>
@@ -364,21 +361,6 @@ __global__ void __launch_bounds__(TPB) k_mass(const BlockDev b, const int* __res
   (void)err;
 }
 
-bool g_pairs_ready = false;
-void init_pairs() {
-  if (g_pairs_ready) return;
-  unsigned char p10[55][2], p27[378][2];
-  int k = 0;
-  for (int J = 0; J < 10; ++J)
-    for (int I = J; I < 10; ++I) { p10[k][0] = (unsigned char)I; p10[k][1] = (unsigned char)J; ++k; }
-  k = 0;
-  for (int J = 0; J < 27; ++J)
-    for (int I = J; I < 27; ++I) { p27[k][0] = (unsigned char)I; p27[k][1] = (unsigned char)J; ++k; }
-  HOEFEM_CUDA(cudaMemcpyToSymbol(c_pairs10, p10, sizeof(p10)));
-  HOEFEM_CUDA(cudaMemcpyToSymbol(c_pairs27, p27, sizeof(p27)));
-  g_pairs_ready = true;
-}
-
 }  // namespace
 
 template <int NN, class R>
@@ -414,7 +396,6 @@ void launch_stiffness_kind(const Model& m, const Block& blk, const MatDev& mat, 
 // e * (3 nn)^2), no scatter.
 void launch_stiffness_staged(const Model& m, const Block& blk, const MatDev& mat, const double* u, double* stage,
                              cudaStream_t s) {
-  init_pairs();
   if (blk.kind == HOEFEM_ELEM_TET10) launch_stiffness_kind<10, double>(m, blk, mat, u, nullptr, s, stage);
   else if (blk.ne > 0) launch_stiffness_hex27(m, blk, nullptr, (int)blk.ne, mat, u, nullptr, stage, nullptr, s);
   HOEFEM_CUDA(cudaGetLastError());
@@ -422,7 +403,6 @@ void launch_stiffness_staged(const Model& m, const Block& blk, const MatDev& mat
 
 void launch_stiffness(const Model& m, const MatDev& mat, const double* u, double* vals, cudaStream_t s,
                       int precision, bool assign) {
-  init_pairs();
   const bool f32 = precision == PRECISION_FP32;
   // a single block whose gather writes every entry stores instead of adding
   const bool one = m.blocks.size() == 1;

@@ -34,6 +34,7 @@
 
 #include "element_math.cuh"
 #include "internal.h"
+#include "pair_tables.h"
 
 namespace hoefem {
 
@@ -48,16 +49,7 @@ constexpr int ASE = QT * AS + 2;     // per element: the two elements of a warp 
 constexpr int BSE = NW * 90 + 2;
 constexpr int NPAIR = 55;
 
-// place of a symmetric 4 x 4 index pair x <= y: 00 01 02 03 11 12 13 22 23 33
-__host__ __device__ constexpr int sym4(int x, int y) {
-  const int lo = x < y ? x : y, hi = x < y ? y : x;
-  return 4 * lo - lo * (lo - 1) / 2 + hi - lo;
-}
-
-// Four terms per node pair: offset of the block in the element's array (m * 90
-// + 9 * block), bit 11 set if it is read transposed, and the coefficient + 8
-// above bit 12 (values are multiples of 1: 16 is stored as 7).
-__constant__ int c_terms[NPAIR][4];
+__constant__ MomentTerms c_terms = moment_terms();
 
 __global__ void __launch_bounds__(EPC* TPE, 2) k_stiffness_moments(const BlockDev b, const double* __restrict__ X,
                                                                    const double* __restrict__ u,
@@ -238,7 +230,7 @@ __global__ void __launch_bounds__(EPC* TPE, 2) k_stiffness_moments(const BlockDe
     double w[4];
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
-      const int c = c_terms[p][n], k = (c >> 12) - 8;
+      const int c = c_terms.at[p][n], k = (c >> 12) - 8;
       w[n] = (double)(k == 7 ? 16 : k);
       at[n][0] = (c & 2047) + (c & 2048 ? i : 3 * i);
       at[n][1] = c & 2048 ? 3 : 1;
@@ -259,45 +251,6 @@ __global__ void __launch_bounds__(EPC* TPE, 2) k_stiffness_moments(const BlockDe
   if (active && sub == 0 && !s_ok[el]) set_error(err, HOEFEM_ERR_SINGULAR);
 }
 
-void init_terms() {
-  static std::atomic<bool> ready[64];
-  int dev = 0;
-  HOEFEM_CUDA(cudaGetDevice(&dev));
-  if (dev >= 0 && dev < 64 && ready[dev].load()) return;
-  static const int edge[6][2] = {{0, 1}, {1, 2}, {0, 2}, {0, 3}, {2, 3}, {1, 3}};
-  int t[NPAIR][4];
-  // coefficient c times the (x, y) block of weight m
-  auto term = [](int m, int x, int y, int c) {
-    return (m * 90 + 9 * sym4(x, y)) | (x > y ? 2048 : 0) | (((c == 16 ? 7 : c) + 8) << 12);
-  };
-  int p = 0;
-  for (int J = 0; J < 10; ++J)
-    for (int I = J; I < 10; ++I, ++p) {
-      if (I < 4) {  // (4 l_I - 1) (4 l_J - 1)
-        t[p][0] = term(sym4(I, J), I, J, 16);
-        t[p][1] = term(10 + I, I, J, -4);
-        t[p][2] = term(10 + J, I, J, -4);
-        t[p][3] = term(14, I, J, 1);
-        continue;
-      }
-      const int a = edge[I - 4][0], d = edge[I - 4][1];
-      if (J < 4) {  // 4 (l_d g_a + l_a g_d), (4 l_J - 1) g_J
-        t[p][0] = term(sym4(d, J), a, J, 16);
-        t[p][1] = term(10 + d, a, J, -4);
-        t[p][2] = term(sym4(a, J), d, J, 16);
-        t[p][3] = term(10 + a, d, J, -4);
-      } else {
-        const int f = edge[J - 4][0], h = edge[J - 4][1];
-        t[p][0] = term(sym4(d, h), a, f, 16);
-        t[p][1] = term(sym4(d, f), a, h, 16);
-        t[p][2] = term(sym4(a, h), d, f, 16);
-        t[p][3] = term(sym4(a, f), d, h, 16);
-      }
-    }
-  HOEFEM_CUDA(cudaMemcpyToSymbol(c_terms, t, sizeof(t)));
-  if (dev >= 0 && dev < 64) ready[dev].store(true);
-}
-
 }  // namespace
 
 bool stiffness_moments_eligible(const Block& blk) {
@@ -307,7 +260,6 @@ bool stiffness_moments_eligible(const Block& blk) {
 // The block's node-pair blocks pblk[(e 55 + p) 9 + 3 i + j] (FP64).
 void launch_stiffness_moments(const Model& m, const Block& blk, const MatDev& mat, const double* u, double* pblk,
                               cudaStream_t s) {
-  init_terms();
   if (!blk.d_moment_w.p) {
     std::vector<double> w(blk.qw.size() * 16, 0.0);
     for (size_t q = 0; q < blk.qw.size(); ++q) {
