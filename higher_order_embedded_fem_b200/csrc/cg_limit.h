@@ -1,6 +1,7 @@
-// When a CG solve ends.  Host code without CUDA types (the device takes the
-// same functions), so that the ends can be tested on the CPU: a kernel that runs
-// a whole solve in one launch must not depend on the host to stop it.
+// The scalar rules of the CG kernels: when a solve ends, and which sums of the next
+// residual are formed ahead of it.  Host code without CUDA types (the device takes
+// the same functions), so that they can be tested on the CPU: a kernel that runs a
+// whole solve in one launch must not depend on the host to stop it.
 #pragma once
 
 #include <cmath>
@@ -49,6 +50,16 @@ HOEFEM_HD inline bool cg_iteration_end(double alpha, double rr, double tol, doub
   if (iters < limit) return false;
   status = HOEFEM_CG_MAX_ITERATIONS;
   return true;
+}
+
+// r'.r' of r' = r - alpha A p from r.r, r.Ap and Ap.Ap (or z'.r' from the same sums
+// with the diagonal); false where they cancel.  The three terms are at most of the
+// size of 4 r.r there, so the relative error is about 4 r.r / r'.r' roundings: a
+// drop of up to 10 costs one digit (1e-14).  A lower bar would cost as many digits
+// as it allows the sum to drop.
+HOEFEM_HD inline bool cg_next_sum(double alpha, double rr, double rap, double apap, double& next) {
+  next = rr - 2.0 * alpha * rap + alpha * alpha * apap;
+  return next > 0.1 * rr;
 }
 
 }  // namespace hoefem

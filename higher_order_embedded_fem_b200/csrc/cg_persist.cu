@@ -37,9 +37,10 @@
 //  3. x, r and p = z + beta p of the CTA's nodes
 // With the diagonal or no preconditioner (two barriers): phase 1 also sums
 // r.r, r.Ap, Ap.Ap and the same with D, from which r'.r' and z'.r' of the
-// updated residual follow without a second pass; where they drop by more than
-// 1e4 in one step (cancellation), the sums are formed from the updated
-// residual instead, with a barrier of their own.
+// updated residual follow without a second pass, to 1e-14; where they drop by more
+// than 10 in one step (cancellation, cg_next_sum), the sums are formed from the
+// updated residual instead, with a barrier of their own.  r itself is updated as
+// ever and its sums are formed anew in every iteration, so nothing accumulates.
 // Deterministic: the tile split, the order inside a warp, over warps and over
 // CTAs are all fixed.
 //
@@ -586,9 +587,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_pcg(const Args A) {
       rr = sum[0];
       zr = sum[1];
     } else {
-      rr = sum[1] - 2.0 * alpha * sum[2] + alpha * alpha * sum[3];
-      zr = PK == 1 ? sum[4] - 2.0 * alpha * sum[5] + alpha * alpha * sum[6] : rr;
-      if (!(rr > 1e-4 * sum[1]) || !(zr > 1e-4 * zTr)) {
+      bool formed = cg_next_sum(alpha, sum[1], sum[2], sum[3], rr);
+      zr = rr;
+      if (PK == 1) formed = cg_next_sum(alpha, sum[4], sum[5], sum[6], zr) && formed;
+      if (!formed) {
         double racc = 0.0, zacc = 0.0;
         for (int a = na + (int)threadIdx.x; a < nb; a += WORKERS)
 #pragma unroll
