@@ -73,7 +73,13 @@ constexpr int NWARP = 15;              // consumer warps (with the producer 512 
 constexpr int WORKERS = 32 * NWARP;
 constexpr int THREADS = WORKERS + 32;  // and the producer warp
 constexpr int MAX_STAGES = 32;         // one producer lane each
-constexpr int IDX_BYTES = 160;  // row offsets (33 + 3 ints) or a subdomain's node list, 16-byte granules
+// Row offsets of a tile or node list of a subdomain (its slots go where a tile's
+// neighbours do), from up to three ints ahead: 16-byte granules.
+constexpr int IDX_BYTES = 160;
+static_assert(IDX_BYTES % 16 == 0 && IDX_BYTES >= (4 * (3 + PCG_MAX_TILE_NODES + 1) + 15) / 16 * 16 &&
+                  IDX_BYTES >= (4 * (3 + PCG_MAX_SUB_NODES) + 15) / 16 * 16,
+              "the lists fit their part of a stage");
+static_assert(3 * PCG_MAX_SUB_NODES <= 96, "a block's columns in three per lane");
 constexpr int TILE_COST = 4096;  // bytes a tile's latency is worth in the CTA split
 constexpr int MAX_G = 256;      // CTAs the barrier's readers cover (8 entries a lane)
 constexpr size_t SMEM_BUDGET = 192 * 1024;  // the rest stays L1 for the gathers of p
@@ -414,7 +420,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_pcg(const Args A) {
     for (int k = 0; k < MAX_SUMS; ++k) acc[k] = 0.0;
     // node and component this lane's exchange ends with (the others double one)
     const int on = lane / (32 / NG), oc = lane & (16 / NG) ? 2 : (lane & (8 / NG) ? 1 : 0);
-    const bool owner = NG == 8 ? (lane & 3) != 3 : !(lane & 1) && (lane & 6) != 6;
+    const bool owner = !(lane & 1) && (lane & 6) != 6;
     run_items(nop, [&](unsigned char* stg) {
       const PcgTile T = *reinterpret_cast<const PcgTile*>(stg);
       const int* off = reinterpret_cast<const int*>(stg + 32) + (T.n0 & 3);
@@ -483,7 +489,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_pcg(const Args A) {
         X s0 = (u2 ? v[0][2] : v[0][0]) + __shfl_xor_sync(0xffffffffu, u2 ? v[0][0] : v[0][2], B2);
         const X s1 = v[0][1] + __shfl_xor_sync(0xffffffffu, v[0][1], B2);
         s0 = (!u2 && u1 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, u2 || u1 ? s0 : s1, B1);
-        if (NG == 4) s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
+        s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
         if (mine) {
           const double t = (double)s0;
           A.Ap[dof] = t;
@@ -722,7 +728,7 @@ bool cg_persist_usable(CgWork& w, const void* vals, bool f32, const Precond* P, 
   Model& m = *w.m;
   if (w.on_chunk || m.spmv_pinned || m.nv == 0 || ((uintptr_t)vals & 15)) return false;
   const bool sw = P && P->kind == PREC_SCHWARZ;
-  if (sw && (!P->block_apply || P->apply_pinned || P->nsub == 0 || 3 * P->max_nodes > 96)) return false;
+  if (sw && (!P->block_apply || P->apply_pinned || P->nsub == 0 || P->max_nodes > PCG_MAX_SUB_NODES)) return false;
   int dev = 0, coop = 0;
   HOEFEM_CUDA(cudaGetDevice(&dev));
   HOEFEM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));

@@ -23,7 +23,8 @@ struct alignas(16) PcgSwTile {
   int o, dim, row0, rows, pad0, pad1;
 };
 
-constexpr int PCG_MAX_TILE_NODES = 16;  // bounds a tile's row offsets and own vector entries
+constexpr int PCG_MAX_TILE_NODES = 16;  // bounds a tile's row offsets in a stage
+constexpr int PCG_MAX_SUB_NODES = 32;   // bounds a subdomain's node list in a stage, and its rows in three per lane
 constexpr int PCG_SW_ROWS = 8;          // Schwarz rows reduced together
 
 // Bytes of the 16-byte granules that cover [begin, end) bytes, not reaching
