@@ -281,8 +281,7 @@ __global__ void __launch_bounds__((NT * NT + 31) / 32 * 32) k_schwarz_gj(
 __global__ void __launch_bounds__(FACTOR_TPB) k_schwarz_factor(
     const int* __restrict__ fallback, const int* __restrict__ sub_off, const int* __restrict__ sub_nodes,
     const long long* __restrict__ gmap_off, const int* __restrict__ gmap, const int* __restrict__ adj_off, const long long* __restrict__ jbase,
-    const double* __restrict__ J, const long long* __restrict__ stage_off, double* __restrict__ stage,
-    double* __restrict__ sym, int* err) {
+    const double* __restrict__ J, const long long* __restrict__ stage_off, double* __restrict__ sym, int* err) {
   if ((int)blockIdx.x >= fallback[0]) return;
   extern __shared__ double smem[];
   const int sidx = fallback[1 + blockIdx.x];
@@ -318,7 +317,6 @@ __global__ void __launch_bounds__(FACTOR_TPB) k_schwarz_factor(
     V[k] = (r == c) ? 1.0 : 0.0;
   }
   __syncthreads();
-  double* out = stage + stage_off[sidx];
 
   // ---- general path: cyclic Jacobi eigen-decomposition -------------------------
   jacobi_eigen_block(A, V, cs, sn, m, dim, s_red);
@@ -346,17 +344,17 @@ __global__ void __launch_bounds__(FACTOR_TPB) k_schwarz_factor(
   if (!(s_red[0] > 0.0) || !isfinite(s_red[0])) {
     if (threadIdx.x == 0) atomicCAS(err, 0, HOEFEM_ERR_NONFINITE);
   }
-  // recompose P = V f V^T into the staging buffer (row-major dim x dim)
+  // the symmetric part of P = V f V^T (whose two halves differ in rounding)
+  double* out = sym + stage_off[sidx];
   for (int k = threadIdx.x; k < dim * dim; k += blockDim.x) {
-    int i = k / dim, j = k % dim;
-    double s = 0.0;
-    for (int t = 0; t < dim; ++t) s += V[i * m + t] * A[t * m + t] * V[j * m + t];
-    out[k] = s;
-  }
-  __syncthreads();  // the block's own writes
-  for (int k = threadIdx.x; k < dim * dim; k += blockDim.x) {
-    const int r = k / dim, c = k % dim;
-    sym[stage_off[sidx] + k] = 0.5 * (out[k] + out[c * dim + r]);
+    const int i = k / dim, j = k % dim;
+    double s = 0.0, r = 0.0;
+    for (int t = 0; t < dim; ++t) {
+      const double vi = V[i * m + t], vj = V[j * m + t], f = A[t * m + t];
+      s += vi * f * vj;
+      r += vj * f * vi;
+    }
+    out[k] = 0.5 * (s + r);
   }
 }
 
@@ -571,7 +569,6 @@ void precond_create_schwarz(Precond& p, const i64* sub_off, const i64* sub_nodes
   }
   p.vals.alloc(p.nnz);
   p.vals.zero(st);
-  p.staging.alloc(stage_off[nsub]);
   p.d_err.alloc(1);
   p.d_fallback.alloc(1 + nsub);
   p.d_sched.alloc(2);
@@ -642,7 +639,7 @@ void precond_update(Precond& p, const double* J, cudaStream_t s) {
     (note_launch(), k_schwarz_factor<<<(int)p.nsub, FACTOR_TPB, smem, s>>>(p.d_fallback.p, p.d_sub_off.p,
                                                                            p.d_sub_nodes.p, p.d_gmap_off.p, p.d_gmap.p,
                                                                            m.d_adj_off.p, m.d_base.p, J, p.d_stage_off.p,
-                                                                           p.staging.p, p.bsym.p, p.d_err.p));
+                                                                           p.bsym.p, p.d_err.p));
     HOEFEM_CUDA(cudaGetLastError());
     if (!lazy) scatter_blocks(p, s);
   }

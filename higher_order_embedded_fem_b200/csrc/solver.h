@@ -35,7 +35,7 @@ struct Precond {
   DBuf<int> d_adj_off, d_adj, d_diag_slot, d_sub_off, d_sub_nodes, d_gmap, d_smap, d_color_subs, d_untreated;
   DBuf<long long> d_base, d_gmap_off;
   DBuf<unsigned char> d_diag_only;
-  DBuf<double> vals, staging;  // staging: the fallback's recomposed blocks
+  DBuf<double> vals;
   DBuf<float> vals32;  // FP32 copy of the Schwarz values (mixed-precision apply)
   bool want_fp32 = false;
   DBuf<long long> d_stage_off;
@@ -48,8 +48,8 @@ struct Precond {
   bool spmv_pinned = false;  // set explicitly by the caller: no autotuning
   DBuf<int> d_tnodes;      // nodes with subdomain rows (the rest are untreated, diagonal only)
   i64 tnodes_count = 0;
-  // Block apply (CG): the symmetrized inverted subdomain blocks (staging
-  // layout) applied as dense products into ysub (3 entries per subdomain
+  // Block apply (CG): the symmetrized inverted subdomain blocks (row-major, at
+  // d_stage_off) applied as dense products into ysub (3 entries per subdomain
   // node), then summed per node over its subdomains in subdomain order.
   bool block_apply = true;
   bool apply_pinned = false;  // the apply was chosen by the caller (hoefem_precond_set_block_apply)
