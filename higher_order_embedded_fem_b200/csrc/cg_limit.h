@@ -35,18 +35,29 @@ inline long long cg_chunks_of(long long iterations, long long chunk) {
   return iterations > 0 ? iterations / chunk + (iterations % chunk != 0) : 1;
 }
 
-// The end of an iteration with step `alpha` and squared residual `rr` after it:
-// counts it and decides whether the solve is over (status set if so).  With
-// alpha a NaN every entry of x and r is NaN from here on, so no later iteration
-// can change the outcome: the solve ends as it would at its limit.
-HOEFEM_HD inline bool cg_iteration_end(double alpha, double rr, double tol, double bnorm, long long limit,
-                                       long long& iters, int& status) {
+// Whether an iteration takes its step alpha = zTr / pAp; the solve is over (status
+// set) if not.  With a NaN among the two, every entry of x and r is NaN after the
+// step, so no later iteration can change the outcome: this one counts as the last
+// that the limit allows.  (One test while all is well.)
+HOEFEM_HD inline bool cg_step_begin(double pAp, double zTr, long long limit, long long& iters, int& status) {
+  if (pAp > 0.0 && zTr > 0.0) return true;
+  if (pAp <= 0.0 || zTr <= 0.0) {
+    status = pAp <= 0.0 ? HOEFEM_CG_INDEFINITE_OPERATOR : HOEFEM_CG_INDEFINITE_PRECONDITIONER;
+    return false;
+  }
+  iters = limit - 1;
+  return true;
+}
+
+// The end of an iteration with the squared residual `rr`: counts it, and whether the
+// solve is over (status set).
+HOEFEM_HD inline bool cg_iteration_end(double rr, double tol, double bnorm, long long limit, long long& iters,
+                                       int& status) {
   iters += 1;
   if (sqrt(rr) <= tol * bnorm) {
     status = HOEFEM_OK;
     return true;
   }
-  if (alpha != alpha) iters = limit;
   if (iters < limit) return false;
   status = HOEFEM_CG_MAX_ITERATIONS;
   return true;

@@ -514,9 +514,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_pcg(const Args A) {
     pAp = sum[0];
     if (PK == 1) zTr = sum[4];
     if (PK == 0) zTr = sum[1];
-    if (pAp <= 0.0 || zTr <= 0.0) {
+    if (!cg_step_begin(pAp, zTr, limit, iters, status)) {
       done = 1;
-      status = pAp <= 0.0 ? HOEFEM_CG_INDEFINITE_OPERATOR : HOEFEM_CG_INDEFINITE_PRECONDITIONER;
       break;
     }
     alpha = zTr / pAp;
@@ -617,7 +616,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_pcg(const Args A) {
         stepped = true;
       }
     }
-    if (cg_iteration_end(alpha, rr, tol, bnorm, limit, iters, status)) {
+    if (cg_iteration_end(rr, tol, bnorm, limit, iters, status)) {
       done = 1;
     } else {
       beta = zr / zTr;

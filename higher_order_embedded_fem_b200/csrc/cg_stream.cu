@@ -462,9 +462,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_cg_stream(Args A) {
     pipe::named_sync(1, CONSUMERS);
     tock(3, tb);
     pAp = s_bc[0];
-    if (pAp <= 0.0 || zTr <= 0.0) {
+    if (!cg_step_begin(pAp, zTr, limit, iters, status)) {
       done = 1;
-      status = pAp <= 0.0 ? HOEFEM_CG_INDEFINITE_OPERATOR : HOEFEM_CG_INDEFINITE_PRECONDITIONER;
       pcur = (int)((it + 1) & 1);
       rcur = (int)(it & 1);
       break;
@@ -597,7 +596,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_cg_stream(Args A) {
     ++it;
     pcur = (int)(it & 1);
     rcur = (int)(it & 1);
-    if (cg_iteration_end(alpha, rr, tol, bnorm, limit, iters, status)) {
+    if (cg_iteration_end(rr, tol, bnorm, limit, iters, status)) {
       done = 1;
       break;
     }

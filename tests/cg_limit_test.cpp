@@ -13,11 +13,14 @@ static int fail(const char* what) {
   return 1;
 }
 
-// One launch: iterations with the given step and squared residual until the end;
+// One launch: iterations with the given p.Ap, z.r and squared residual until the end;
 // false if it has not ended after `most` of them.
-static bool launch(double alpha, double rr, double tol, long long limit, long long& iters, int& status, long long most) {
-  for (long long k = 0; k < most; ++k)
-    if (cg_iteration_end(alpha, rr, tol, 1.0, limit, iters, status)) return true;
+static bool launch(double pAp, double zTr, double rr, double tol, long long limit, long long& iters, int& status,
+                   long long most) {
+  for (long long k = 0; k < most; ++k) {
+    if (!cg_step_begin(pAp, zTr, limit, iters, status)) return true;
+    if (cg_iteration_end(rr, tol, 1.0, limit, iters, status)) return true;
+  }
   return false;
 }
 
@@ -43,17 +46,32 @@ int main() {
     const long long limit = cg_iteration_limit(m, 300, 8);
     long long iters = 0;
     int status = HOEFEM_OK;
-    if (!launch(nan, nan, 1e-10, limit, iters, status, 1) || status != HOEFEM_CG_MAX_ITERATIONS || iters != limit)
-      return fail("NaN step");
+    for (double pAp : {nan, 0.5})
+      for (double zTr : {nan, 0.5}) {
+        if (pAp == zTr) continue;
+        iters = 0;
+        status = HOEFEM_OK;
+        if (!launch(pAp, zTr, nan, 1e-10, limit, iters, status, 1) || status != HOEFEM_CG_MAX_ITERATIONS || iters != limit)
+          return fail("NaN step");
+      }
+    // an indefinite operator or preconditioner ends it before the step
+    for (double bad : {0.0, -1.0, -inf}) {
+      iters = 3;
+      if (!launch(bad, nan, 1.0, 1e-10, limit, iters, status, 1) || status != HOEFEM_CG_INDEFINITE_OPERATOR || iters != 3)
+        return fail("operator");
+      if (!launch(nan, bad, 1.0, 1e-10, limit, iters, status, 1) || status != HOEFEM_CG_INDEFINITE_PRECONDITIONER ||
+          iters != 3)
+        return fail("preconditioner");
+    }
     // a residual that never falls (and one that only is a NaN): the limit itself
     for (double rr : {1.0, inf, nan}) {
       iters = 0;
       status = HOEFEM_OK;
-      if (!launch(0.5, rr, 1e-10, limit, iters, status, limit) || status != HOEFEM_CG_MAX_ITERATIONS || iters != limit)
+      if (!launch(0.5, 0.5, rr, 1e-10, limit, iters, status, limit) || status != HOEFEM_CG_MAX_ITERATIONS || iters != limit)
         return fail("limit");
     }
     iters = limit - 1;  // convergence in the last iteration counts
-    if (!launch(0.5, 1e-24, 1e-10, limit, iters, status, 1) || status != HOEFEM_OK || iters != limit) return fail("last");
+    if (!launch(0.5, 0.5, 1e-24, 1e-10, limit, iters, status, 1) || status != HOEFEM_OK || iters != limit) return fail("last");
   }
   // a recurrence that reports convergence after every iteration, refuted by the true
   // residual each time: launches until the chunks are used up
@@ -63,7 +81,7 @@ int main() {
     int status = HOEFEM_OK;
     while (chunks < most && launches <= most) {
       const long long it0 = iters;
-      if (!launch(0.5, 0.0, 1e-17, cg_iteration_limit(-1, 300, 8), iters, status, 1) || status != HOEFEM_OK)
+      if (!launch(0.5, 0.5, 0.0, 1e-17, cg_iteration_limit(-1, 300, 8), iters, status, 1) || status != HOEFEM_OK)
         return fail("claimed convergence");
       chunks += cg_chunks_of(iters - it0, 8);
       ++launches;
