@@ -127,9 +127,9 @@ __device__ __forceinline__ bool inv3_spd(const double* p, double (&o)[9]) {
 // certificate go to the fallback list; the others are stored symmetrized.
 // 27 steps of two barriers instead of 81 of one, and a tile of three nodes makes
 // the pivot's place in it a compile-time one and 243 FMAs follow 54 loads: 1,728
-// blocks of 81 x 81 in 303 us (16 x 16 threads with 6 x 6 entries each, scalar
+// blocks of 81 x 81 in 297 us (16 x 16 threads with 6 x 6 entries each, scalar
 // steps: 432 us and 44 us for the symmetrization; with node steps 483).  Bound
-// by latency: 244 registers leave two CTAs of three warps per SM, and three
+// by latency: 254 registers leave two CTAs of three warps per SM, and three
 // spill (765 us).
 template <int NT>
 __global__ void __launch_bounds__((NT * NT + 31) / 32 * 32) k_schwarz_gj(

@@ -32,6 +32,9 @@
 // pipe (36.9 TFLOP/s measured, against 32.2 of plain FMA loops): 11.7 k
 // multiply-adds per point.  4,608 elements of 8 to 27 points: 458 -> 179 us (of
 // which the products are a third; the rest is latency at two consumer warps per quadrant).
+// Relative error against extended precision 2.8e-16 to 3.1e-16 (cylinders of 8^3 and
+// 6^3 cells) where the pair loop had 4.9e-16 to 4.1e-16: the Jacobian comes from
+// edges, not from absolute coordinates.
 #include <cuda_runtime.h>
 
 #include <algorithm>

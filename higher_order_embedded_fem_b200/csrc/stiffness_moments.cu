@@ -16,8 +16,12 @@
 // 14 x (560 + 45 x 15) + 3,000 operations instead of 55 x 14 x 62, and the pair
 // loop's operands are no longer read from shared memory per pair (31
 // loads for 60 FMAs, which bound it).  201,600 elements: 2.56 -> 0.81 ms (0.8 GB
-// of blocks written; eight warps per SM fit, so it is bound by their latency).
-// Relative error against 64-bit torch 3e-16, as the pair loop's (2e-16).
+// of blocks written).  Bound by shared memory, whose pipe is at 78 % of its peak
+// (FP64 34 %): phase B reads 45 values and a weight for 45 FMAs, and the eight
+// warps per SM that fit do not hide the rest.
+// Relative error against extended precision 3.1e-16 to 3.9e-16 (boxes of 216 and
+// 1,080 elements) where the pair loop has 2.1e-16 to 2.7e-16: the four terms of a
+// pair cancel in part, so the rounding of the moments' sums counts more.
 //
 // Taken for every uniform Tet10 rule in the staged path; the pair loop
 // (k_stiffness) keeps the FP32 blocks, per-element rules, the colored scatter and

@@ -259,7 +259,8 @@ class NewtonCgIntegrator3d:
 
     def set_cg_engine(self, engine="auto", schwarz_fp16=False, phase_profile=False):
         """CG engine of the Jacobian solves: "auto" (the faster engine, timed
-        on the first solves), "chunked" (CUDA graphs of kernel chunks) or
+        on the first solves), "chunked" (one persistent launch on the CSR values,
+        or CUDA graphs of kernel chunks where that does not apply) or
         "streamed" (persistent streamed CG; error if it cannot run);
         schwarz_fp16 keeps the Schwarz blocks of the mixed form in scaled FP16;
         phase_profile records per-phase times (hoefem_integrator_set_cg_engine)."""

@@ -132,8 +132,10 @@ int hoefem_model_autotune(hoefem_model m, int32_t* lanes);
    (neighbour-major), or 108, 116, 132 (the same lane counts, column-streaming
    traversal), for FP64 and FP32 values, and turns the automatic choice off.
    Otherwise hoefem_model_autotune / integrator set-up time the variants on
-   the SpMV alone, and the first CG solves time candidate pairs (operator,
-   Schwarz apply) chunk by chunk per value precision and keep the fastest. */
+   the SpMV alone, and CG solves that run as graphs of kernel chunks time candidate
+   pairs (operator, Schwarz apply) chunk by chunk per value precision and keep the
+   fastest.  An explicit variant keeps the CG on the graphs
+   (hoefem_model_set_cg_engine). */
 int hoefem_model_set_spmv_variant(hoefem_model m, int32_t variant);
 /* The SpMV variants in use for FP64 and FP32 operator values. */
 int hoefem_model_get_spmv_variants(hoefem_model m, int32_t* fp64_values, int32_t* fp32_values);
@@ -254,7 +256,9 @@ int hoefem_precond_nnz(hoefem_precond p, int64_t* nnz);
    reference applies the assembled CSR matrix with MKL): on (default) = the
    symmetrized inverted subdomain blocks as dense products, summed per node in
    subdomain order; off = SpMV over the assembled values.  Both are P r; they
-   differ only in rounding.  hoefem_precond_apply always uses the CSR. */
+   differ only in rounding.  Either choice by this call keeps the CG on the
+   graphs of kernel chunks (hoefem_model_set_cg_engine).  hoefem_precond_apply
+   applies the blocks too, or the CSR once it has been assembled. */
 int hoefem_precond_set_block_apply(hoefem_precond p, int32_t on);
 /* SpMV variant of the Schwarz apply (as hoefem_model_set_spmv_variant);
    chosen by the autotuner at creation and by the CG's online choice
