@@ -89,7 +89,8 @@ __device__ __forceinline__ bool inv3_spd(const double* p, double (&o)[9]) {
   const double det = p[0] * o[0] + p[1] * o[3] + p[2] * o[6];
   // signs and exponents by the high words (integer tests, off the FP64 chain); a
   // determinant near either end of the exponents is left to the elimination
-  const int far = __double2hiint(__fma_rn(-0.25 * p[0], p[4] * p[8], det));
+  // (no product of its own shared with the minors, whose rounding would follow)
+  const int far = __double2hiint(__fma_rn(-p[0], (0.25 * p[4]) * p[8], det));
   const unsigned size = (unsigned)__double2hiint(det) - (unsigned)((1023 - 660) << 20);
   if (min(min(__double2hiint(p[0]), __double2hiint(o[8])), far) > 0 && size < (unsigned)((2 * 660) << 20)) {
     const double inv = 1.0 / det;
